@@ -18,6 +18,8 @@
 
 #include <cstdint>
 
+#include "exact64.cuh"
+
 namespace als {
 
 enum Recon { RECON_NONE = 0, RECON_WENO2 = 1, RECON_ENO2 = 2, RECON_ENO3 = 3, RECON_ENO4 = 4,
@@ -414,6 +416,44 @@ __device__ __forceinline__ R twice_reciprocal(R d, R recip) {
     return out;
 }
 
+// WENO2 weights (w0Left, w1Left, w0Right, w1Right) from the smoothness
+// denominators d0 = 3 (eps + b0)^2, d1 = 3 (eps + b1)^2, as reconstruct_f
+// forms them; the compiler's division.
+static __device__ __noinline__ double4 weno2_weights_plain(double d0, double d1) {
+    const double a0Left = 1.0 / d0;
+    const double a1Right = 1.0 / d1;
+    const double a1Left = twice_reciprocal(d1, a1Right);
+    const double a0Right = twice_reciprocal(d0, a0Left);
+    double4 w;
+    w.x = a0Left / (a0Left + a1Left);
+    w.y = a1Left / (a0Left + a1Left);
+    w.z = a0Right / (a0Right + a1Right);
+    w.w = a1Right / (a0Right + a1Right);
+    return w;
+}
+
+// d0, d1 >= 3e-16 by construction; below 2^400 every intermediate is normal.
+__device__ __forceinline__ double4 weno2_weights(double d0, double d1) {
+    const unsigned top = max(unsigned(__double2hiint(d0)), unsigned(__double2hiint(d1)));
+    if (top >= unsigned(hi_pow2(400))) {
+        return weno2_weights_plain(d0, d1);
+    }
+    const double a0Left = rcp64(d0);
+    const double a1Right = rcp64(d1);
+    const double a1Left = 2.0 * a1Right;
+    const double a0Right = 2.0 * a0Left;
+    const double sl = a0Left + a1Left;
+    const double sr = a0Right + a1Right;
+    const double yl = rcp64(sl);
+    const double yr = rcp64(sr);
+    double4 w;
+    w.x = quot64(a0Left, sl, yl);
+    w.y = quot64(a1Left, sl, yl);
+    w.z = quot64(a0Right, sr, yr);
+    w.w = quot64(a1Right, sr, yr);
+    return w;
+}
+
 // sign and minmod (alsfvm/include/alsfvm/reconstruction/sign.hpp,
 // minmod.hpp): sign is 1, 0 or -1; minmod is sign(a) times the smallest
 // magnitude when all signs agree, else 0.
@@ -529,14 +569,11 @@ __device__ __forceinline__ void reconstruct_f(const Fetch& f, R* left, R* right,
             w0Right = R(2) * d1 * rr;
             w1Right = d0 * rr;
         } else {
-            const R a0Left = R(1) / d0;
-            const R a1Right = R(1) / d1;
-            const R a1Left = twice_reciprocal(d1, a1Right);
-            const R a0Right = twice_reciprocal(d0, a0Left);
-            w0Left = a0Left / (a0Left + a1Left);
-            w1Left = a1Left / (a0Left + a1Left);
-            w0Right = a0Right / (a0Right + a1Right);
-            w1Right = a1Right / (a0Right + a1Right);
+            const double4 w = weno2_weights(d0, d1);
+            w0Left = w.x;
+            w1Left = w.y;
+            w0Right = w.z;
+            w1Right = w.w;
         }
         const R cl = R(3) * w0Left + w1Left;
         const R cr = R(3) * w1Right + w0Right;
@@ -624,14 +661,11 @@ __device__ __forceinline__ void reconstruct_f(const Fetch& f, R* left, R* right,
             w0Right = R(2) * d1 * rr;
             w1Right = d0 * rr;
         } else {
-            const R a0Left = R(1) / d0;
-            const R a1Right = R(1) / d1;
-            const R a1Left = twice_reciprocal(d1, a1Right);
-            const R a0Right = twice_reciprocal(d0, a0Left);
-            w0Left = a0Left / (a0Left + a1Left);
-            w1Left = a1Left / (a0Left + a1Left);
-            w0Right = a0Right / (a0Right + a1Right);
-            w1Right = a1Right / (a0Right + a1Right);
+            const double4 w = weno2_weights(d0, d1);
+            w0Left = w.x;
+            w1Left = w.y;
+            w0Right = w.z;
+            w1Right = w.w;
         }
         R rho[3], u[3][NSD], p[3];
 #pragma unroll

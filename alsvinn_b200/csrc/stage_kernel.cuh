@@ -22,7 +22,7 @@
 // the state and no stage waits on the host.
 #pragma once
 
-#include "euler_math.cuh"
+#include "euler_exact64.cuh"
 #include "stage_params.h"
 
 namespace als {
@@ -405,7 +405,7 @@ __device__ __forceinline__ void stage_direction(const GridDesc& gd, R gamma, con
                 ul[v] = rec[(NV + v) * RC + rl];
                 ur[v] = rec[v * RC + rr];
             }
-            w = face_flux<R, DIM, FLUX, D>(ul, ur, gamma, F);
+            w = face_flux_best<R, DIM, FLUX, D>(ul, ur, gamma, F);
         }
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -645,21 +645,18 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const LevelDesc
         const int bx = b % Lay::BX;
         const int by = (b / Lay::BX) % Lay::BY;
         const int bz = b / (Lay::BX * Lay::BY);
-        const int px = x0 + bx + sh;
-        const int py = DIM > 1 ? y0 + by + sh : 0;
-        const int pz = DIM > 2 ? z0 + bz + sh : 0;
-        const bool inside = px < gd.N[0] && py < gd.N[1] && pz < gd.N[2];
-        const long long idx = inside ? ((long long)pz * gd.N[1] + py) * gd.N[0] + px : 0;
+        // cells beyond the planes read the last column, row or plane: ordinary
+        // values, whose results nobody uses
+        const int px = min(x0 + bx + sh, gd.N[0] - 1);
+        const int py = DIM > 1 ? min(y0 + by + sh, gd.N[1] - 1) : 0;
+        const int pz = DIM > 2 ? min(z0 + bz + sh, gd.N[2] - 1) : 0;
+        const long long idx = ((long long)pz * gd.N[1] + py) * gd.N[0] + px;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            R val = R(0);
-            if (inside) {
-                if (KIND == KIND_RK2_1 || KIND == KIND_RK3_1) {
-                    val = inp(v)[idx] * c;
-                    val = val + unp(v)[idx];
-                } else {
-                    val = inp(v)[idx];
-                }
+            R val = inp(v)[idx];
+            if (KIND == KIND_RK2_1 || KIND == KIND_RK3_1) {
+                val = val * c;
+                val = val + unp(v)[idx];
             }
             box[v * Lay::BOX + b] = val;
         }

@@ -109,7 +109,7 @@ __device__ __forceinline__ void plane_direction(const GridDesc& gd, R gamma, con
             ul[v] = rec[(NV + v) * RC + rl];
             ur[v] = rec[v * RC + rr];
         }
-        const R w = face_flux<R, 3, FLUX, D>(ul, ur, gamma, F);
+        const R w = face_flux_best<R, 3, FLUX, D>(ul, ur, gamma, F);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             flx[v * FC + i] = F[v];
@@ -197,25 +197,21 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
     auto slot = [&](int k) { return ring + ((k - k0 + 3) % 3) * (NV * Lay::PLANE); };
     auto load_plane = [&](int k) {
         R* dst = slot(k);
-        const int pz = k + gd.ghosts;
-        const bool zin = pz >= 0 && pz < gd.N[2];
+        // cells beyond the planes read the nearest column, row or plane:
+        // ordinary values, whose results nobody uses
+        const int pz = max(0, min(k + gd.ghosts, gd.N[2] - 1));
         for (int b = tid; b < Lay::PLANE; b += Lay::THREADS) {
             const int bx = b % Lay::BX;
             const int by = b / Lay::BX;
-            const int px = x0 + bx + sh;
-            const int py = y0 + by + sh;
-            const bool inside = zin && px < gd.N[0] && py < gd.N[1];
-            const long long idx = inside ? ((long long)pz * gd.N[1] + py) * gd.N[0] + px : 0;
+            const int px = min(x0 + bx + sh, gd.N[0] - 1);
+            const int py = min(y0 + by + sh, gd.N[1] - 1);
+            const long long idx = ((long long)pz * gd.N[1] + py) * gd.N[0] + px;
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                R val = R(0);
-                if (inside) {
-                    if (KIND == KIND_RK2_1 || KIND == KIND_RK3_1) {
-                        val = inp(v)[idx] * c;
-                        val = val + unp(v)[idx];
-                    } else {
-                        val = inp(v)[idx];
-                    }
+                R val = inp(v)[idx];
+                if (KIND == KIND_RK2_1 || KIND == KIND_RK3_1) {
+                    val = val * c;
+                    val = val + unp(v)[idx];
                 }
                 dst[v * Lay::PLANE + b] = val;
             }
@@ -262,7 +258,7 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
             for (int v = 0; v < NV; ++v) {
                 rb[v] = Rk[v * Lay::COLS];
             }
-            const R w = face_flux<R, 3, FLUX, 2>(rb, l, gamma, F);
+            const R w = face_flux_best<R, 3, FLUX, 2>(rb, l, gamma, F);
             if (KIND == KIND_FLUX0 && in_region && wmax[2] < w) {
                 wmax[2] = w;
             }
@@ -296,7 +292,7 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
             for (int v = 0; v < NV; ++v) {
                 rb[v] = Rk[v * Lay::COLS];
             }
-            const R w = face_flux<R, 3, FLUX, 2>(rb, l, gamma, Fp);
+            const R w = face_flux_best<R, 3, FLUX, 2>(rb, l, gamma, Fp);
             if (KIND == KIND_FLUX0 && in_region && wmax[2] < w) {
                 wmax[2] = w;
             }
