@@ -220,6 +220,142 @@ __global__ void __launch_bounds__(kThreads) structure_kernel(const T* __restrict
     }
 }
 
+// The cube statistic from a staged box, for H <= HM (2-D and 3-D).
+//
+// structure_kernel above loads a neighbour for every difference; here a block
+// stages its tile and the H - 1 cells around it in shared memory, as FP64
+// and with the boundary applied once, and a thread holds four cells of a
+// column along y: the values above and below them at one (x, z) offset are
+// loaded once and serve every y offset of all four, 0.2 to 0.4 loads per
+// difference, so the two FP64 operations of a difference are what binds.
+// On a torus |u(x) - u(x + d)| summed over all x is the same for d and -d:
+// with periodic boundaries one of each pair is walked and counted twice.
+// 32 x 256^2 FP32 states, H = 8, p = 1, periodic: 1.46 -> 0.36 ms (0.94e9
+// differences, 2.6e12 a second; the FP64 pipe's bound is 9.3e12).
+template<int DIM> struct CubeTile;
+// The largest tile; the host halves y, then z, until the blocks fill the GPU.
+template<> struct CubeTile<2> { static constexpr int X = 32, Y = 64, Z = 1; };
+template<> struct CubeTile<3> { static constexpr int X = 32, Y = 8, Z = 4; };
+
+// SHARE: fewer strips than warps; several warps take one strip and split its
+// x offsets.
+template<class T, int DIM, int BC, int P, int HM, bool SHARE>
+__global__ void __launch_bounds__(kThreads) structure_cube_kernel(const T* __restrict__ states,
+    long long member_stride, StructGeom G, int nvar, int H, double p, double* __restrict__ partial) {
+    constexpr bool HALF = BC == ALS_BC_PERIODIC;
+    constexpr int COLS = 4;              // cells per thread and strip
+    constexpr int W = COLS + 2 * (HM - 1);
+    extern __shared__ double box[];
+    __shared__ double part[kWarps][HM];
+    const int member = blockIdx.z;
+    const int var = blockIdx.y;
+    const int tile = blockIdx.x;
+    const int R = H - 1;
+    const int tx = tile % G.tiles[0];
+    const int ty = (tile / G.tiles[0]) % G.tiles[1];
+    const int tz = tile / (G.tiles[0] * G.tiles[1]);
+    const int x0 = tx * G.tile[0], y0 = ty * G.tile[1], z0 = tz * G.tile[2];
+    const int bx = G.tile[0] + 2 * R;
+    const int by = G.tile[1] + 2 * R;
+    const int bz = DIM > 2 ? G.tile[2] + 2 * R : 1;
+    const T* u = states + (long long)member * member_stride + (long long)var * G.plane;
+    for (int i = threadIdx.x; i < bx * by * bz; i += kThreads) {
+        const int ix = i % bx, iy = (i / bx) % by, iz = i / (bx * by);
+        const int x = bound<BC>(x0 + ix - R, G.n[0]);
+        const int y = bound<BC>(y0 + iy - R, G.n[1]);
+        const int z = DIM > 2 ? bound<BC>(z0 + iz - R, G.n[2]) : 0;
+        box[i] = load(u, ((long long)(z + G.g[2]) * G.N[1] + (y + G.g[1])) * G.N[0] + (x + G.g[0]));
+    }
+    __syncthreads();
+
+    double acc[HM];
+#pragma unroll
+    for (int h = 0; h < HM; ++h) {
+        acc[h] = 0;
+    }
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int strips = G.tile[1] / COLS;         // per plane of the tile
+    const int all = strips * G.tile[2];
+    const int team = SHARE ? warp / all : 0;
+    const int teams = SHARE ? kWarps / all : 1;
+    for (int sidx = SHARE ? warp % all : warp; sidx < all; sidx += kWarps) {
+        const int cy = (sidx % strips) * COLS;
+        const int cz = sidx / strips;
+        const int left = min(COLS, G.n[1] - (y0 + cy));   // cells of the strip inside the grid
+        if (x0 + lane >= G.n[0] || left <= 0 || z0 + cz >= G.n[2]) {
+            continue;
+        }
+        const double* centre = box + ((DIM > 2 ? cz + R : 0) * by + cy + R) * bx + lane + R;
+        double uc[COLS];
+#pragma unroll
+        for (int k = 0; k < COLS; ++k) {
+            uc[k] = centre[k * bx];
+        }
+        for (int dz = DIM > 2 ? (HALF ? 0 : -R) : 0; dz <= (DIM > 2 ? R : 0); ++dz) {
+            for (int dx = (SHARE ? team : 0) - R; dx <= R; dx += SHARE ? teams : 1) {
+                // y offsets from `first`: with HALF and dz = 0 only half the plane
+                const int first = HALF && dz == 0 ? (dx > 0 ? 0 : 1) : -R;
+                const int far = max(abs(dx), abs(dz));
+                const double* col = centre + dz * (by * bx) + dx;
+                double w[W];
+#pragma unroll
+                for (int k = 0; k < W; ++k) {
+                    const int dy = k - (HM - 1);   // row offset from the first cell
+                    w[k] = dy >= first && dy <= R + COLS - 1 ? col[dy * bx] : 0.0;
+                }
+                double near = 0;                  // the offsets whose cube is `far`
+#pragma unroll
+                for (int dy = -(HM - 1); dy <= HM - 1; ++dy) {
+                    if (dy < first || dy > R) {
+                        continue;
+                    }
+                    double d = 0;
+#pragma unroll
+                    for (int k = 0; k < COLS; ++k) {
+                        const double t = spow<P>(fabs(uc[k] - w[k + dy + HM - 1]), p);
+                        d += k < left ? t : 0.0;
+                    }
+                    const int a = dy < 0 ? -dy : dy;
+                    if (a > far) {
+                        acc[a] += d;
+                    } else {
+                        near += d;
+                    }
+                }
+#pragma unroll
+                for (int h = 1; h < HM; ++h) {
+                    if (h == far) {
+                        acc[h] += near;
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 1; h < HM; ++h) {
+        double a = acc[h];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_down_sync(0xffffffffu, a, o);
+        }
+        if (lane == 0) {
+            part[warp][h] = a;
+        }
+    }
+    __syncthreads();
+    const long long row = ((long long)member * nvar + var) * gridDim.x + tile;
+    for (int h = threadIdx.x; h < H; h += kThreads) {
+        double s = 0;
+        if (h > 0) {
+            for (int w = 0; w < kWarps; ++w) {
+                s += part[w][h];
+            }
+        }
+        partial[row * H + h] = HALF ? 2.0 * s : s;
+    }
+}
+
 // out[mv][h] = (sum over tiles, in tile order) / cells
 __global__ void structure_finish(const double* __restrict__ partial, int tiles, int H, long long rows,
     double cells, double* __restrict__ out) {
@@ -236,11 +372,38 @@ __global__ void structure_finish(const double* __restrict__ partial, int tiles, 
     }
 }
 
+// Largest H of the staged cube kernel: its columns of 2 H + 2 values have to
+// stay in registers, and in 3-D its box in shared memory.
+constexpr int kCubeH2 = 8;
+constexpr int kCubeH3 = 6;
+
+__host__ __device__ constexpr bool staged_cube(int dim, bool cube, int H) {
+    return cube && ((dim == 2 && H <= kCubeH2) || (dim == 3 && H <= kCubeH3));
+}
+
 template<class T, int DIM, int BC, int P, bool CUBE>
 cudaError_t launch(const T* states, long long stride, const StructGeom& G, int nvar, int members,
     int direction, int H, double p, double* partial, cudaStream_t s) {
     const int tiles = G.tiles[0] * G.tiles[1] * G.tiles[2];
     dim3 grid(tiles, nvar, members);
+    if constexpr (CUBE && DIM > 1) {
+        if (staged_cube(DIM, CUBE, H)) {
+            constexpr int HM = DIM == 2 ? kCubeH2 : kCubeH3;
+            const int r = 2 * (H - 1);
+            const size_t smem = sizeof(double) * size_t(G.tile[0] + r) * (G.tile[1] + r) *
+                (DIM > 2 ? G.tile[2] + r : 1);
+            const bool share = G.tile[1] / 4 * G.tile[2] < kWarps;
+            auto kernel = share ? structure_cube_kernel<T, DIM, BC, P, HM, true>
+                                : structure_cube_kernel<T, DIM, BC, P, HM, false>;
+            const cudaError_t err = cudaFuncSetAttribute(kernel,
+                cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+            if (err != cudaSuccess) {
+                return err;
+            }
+            kernel<<<grid, kThreads, smem, s>>>(states, stride, G, nvar, H, p, partial);
+            return cudaGetLastError();
+        }
+    }
     structure_kernel<T, DIM, BC, P, CUBE><<<grid, kThreads, 0, s>>>(states, stride, G, nvar,
         direction, H, p, partial);
     return cudaGetLastError();
@@ -318,9 +481,26 @@ extern "C" int als_structure_functions(const als_grid* grid, int boundary, int k
         return ALS_OK;
     }
     const int shapes[3][3] = {{256, 1, 1}, {16, 16, 1}, {8, 8, 4}};
+    const int staged[3][3] = {{0, 0, 0}, {CubeTile<2>::X, CubeTile<2>::Y, CubeTile<2>::Z},
+        {CubeTile<3>::X, CubeTile<3>::Y, CubeTile<3>::Z}};
+    const bool cube = kind == ALS_STRUCTURE_CUBE;
     for (int d = 0; d < 3; ++d) {
-        G.tile[d] = shapes[dim - 1][d];
+        G.tile[d] = (staged_cube(dim, cube, H) ? staged : shapes)[dim - 1][d];
         G.tiles[d] = (G.n[d] + G.tile[d] - 1) / G.tile[d];
+    }
+    if (staged_cube(dim, cube, H)) {
+        // halve the tile along y, then z, while that trims the padded cells by
+        // an eighth or the blocks do not make two per SM
+        auto padded = [&](int d, int t) { return (long long)(G.n[d] + t - 1) / t * t; };
+        auto blocks = [&]() { return (long long)G.tiles[0] * G.tiles[1] * G.tiles[2] * nvar * members; };
+        for (int d = 1; d < dim; ++d) {
+            const int least = d == 1 ? 4 : 1;
+            while (G.tile[d] > least && (8 * padded(d, G.tile[d]) > 9 * padded(d, G.tile[d] / 2) ||
+                                            blocks() < 2 * 148)) {
+                G.tile[d] /= 2;
+                G.tiles[d] = (G.n[d] + G.tile[d] - 1) / G.tile[d];
+            }
+        }
     }
     const long long tiles = (long long)G.tiles[0] * G.tiles[1] * G.tiles[2];
     if (tiles > 0x7fffffffLL) {
