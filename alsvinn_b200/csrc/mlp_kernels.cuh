@@ -9,9 +9,16 @@
 
 namespace mlpk {
 
+// Chunks of K = 64 a CTA holds: the training GEMMs (BN = 64, K <= 256) fit
+// whole; the wide inference tiles keep two, for more CTAs per SM.
+template <int BN>
+__host__ __device__ constexpr int gemm_stages() {
+    return BN == 64 ? 4 : 2;
+}
+
 template <int BN>
 constexpr int gemm_smem_bytes() {
-    return 2 * (kTileM * kChunkK * 2 + BN * kChunkK * 2) + 1024;
+    return gemm_stages<BN>() * (kTileM * kChunkK * 2 + BN * kChunkK * 2) + 1024;
 }
 
 template <int BN, int EPI>
@@ -78,8 +85,9 @@ __device__ __forceinline__ void epilogue16(const GemmArgs& g, long long m, int n
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid) {
     static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "TMEM columns: power of two");
+    constexpr int kStages = gemm_stages<BN>();
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t bars[2];
+    __shared__ uint64_t bars[kStages];
     __shared__ uint64_t drain;
     __shared__ uint32_t tmem_base;
     unsigned char* base = reinterpret_cast<unsigned char*>(
@@ -87,8 +95,8 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
     constexpr int kABytes = kTileM * kChunkK * 2;
     constexpr int kBBytes = BN * kChunkK * 2;
     const unsigned limit = g.wait_limit ? g.wait_limit : kWaitLimit;
-    unsigned char* sa[2] = {base, base + kABytes + kBBytes};
-    unsigned char* sb[2] = {base + kABytes, base + 2 * kABytes + kBBytes};
+    auto sa = [&](int s) { return base + s * (kABytes + kBBytes); };
+    auto sb = [&](int s) { return base + s * (kABytes + kBBytes) + kABytes; };
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -100,8 +108,9 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
         tmem_alloc(&tmem_base, BN);
     }
     if (threadIdx.x == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        for (int k = 0; k < kStages; ++k) {
+            mbar_init(&bars[k], 1);
+        }
         mbar_init(&drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -112,40 +121,63 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
     const uint32_t idesc = instr_desc_bf16(kTileM, BN);
     const int nk = g.K / kChunkK;
 
+    // the MMAs of chunk c from stage st
+    auto issue = [&](int c, int st) {
+        const uint32_t a0 = smem_u32(sa(st));
+        const uint32_t b0 = smem_u32(sb(st));
+#pragma unroll
+        for (int j = 0; j < kChunkK / 16; ++j) {
+            mma_bf16(tmem, smem_desc(a0 + j * 256, 128, 1024),
+                     smem_desc(b0 + j * 256, 128, 1024), idesc, (c > 0 || j > 0) ? 1u : 0u);
+        }
+    };
     int last = -1;          // last chunk whose MMAs were committed
     bool failed = false;
-    for (int c = 0; c < nk; ++c) {
-        const int s = c & 1;
-        bool ok = true;
-        if (c >= 2) {
-            ok = mbar_wait(&bars[s], unsigned((c - 2) >> 1) & 1u, limit);
+    if (nk <= kStages) {
+        for (int c = 0; c < nk; ++c) {
+            stage_operand<kTileM>(sa(c), g.a, m0, kb + c * kChunkK);
+            stage_operand<BN>(sb(c), g.b, n0, kb + c * kChunkK);
         }
-        if (__syncthreads_or(!ok)) {
-            failed = true;
-            break;
-        }
-        stage_operand<kTileM>(sa[s], g.a, m0, kb + c * kChunkK);
-        stage_operand<BN>(sb[s], g.b, n0, kb + c * kChunkK);
-        fence_async_shared();
+        stage_wait();
         __syncthreads();
         if (threadIdx.x == 0) {
             tc_fence_after();
-            const uint32_t a0 = smem_u32(sa[s]);
-            const uint32_t b0 = smem_u32(sb[s]);
-#pragma unroll
-            for (int j = 0; j < kChunkK / 16; ++j) {
-                mma_bf16(tmem, smem_desc(a0 + j * 256, 128, 1024),
-                         smem_desc(b0 + j * 256, 128, 1024), idesc, (c > 0 || j > 0) ? 1u : 0u);
+            for (int c = 0; c < nk; ++c) {
+                issue(c, c);
             }
             if (!g.withhold_commit) {
-                mma_commit(&bars[s]);
+                mma_commit(&bars[0]);
             }
         }
-        last = c;
+        last = 0;           // one commit, on the first barrier
+    } else {
+        for (int c = 0; c < nk; ++c) {
+            const int s = c % kStages;
+            bool ok = true;
+            if (c >= kStages) {
+                ok = mbar_wait(&bars[s], unsigned(c / kStages - 1) & 1u, limit);
+            }
+            if (__syncthreads_or(!ok)) {
+                failed = true;
+                break;
+            }
+            stage_operand<kTileM>(sa(s), g.a, m0, kb + c * kChunkK);
+            stage_operand<BN>(sb(s), g.b, n0, kb + c * kChunkK);
+            stage_wait();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                tc_fence_after();
+                issue(c, s);
+                if (!g.withhold_commit) {
+                    mma_commit(&bars[s]);
+                }
+            }
+            last = c;
+        }
     }
     bool done = false;
     if (last >= 0) {
-        done = mbar_wait(&bars[last & 1], unsigned(last >> 1) & 1u, limit);
+        done = mbar_wait(&bars[last % kStages], unsigned(last / kStages) & 1u, limit);
     }
     if (__syncthreads_or(!done) || failed) {
         if (threadIdx.x == 0) {
@@ -156,10 +188,13 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
         mbar_wait(&drain, 0, kWaitLimit);
     } else {
         tc_fence_after();
-        const long long m = m0 + warp * 32 + lane;
-        const uint32_t lane_base = tmem + (uint32_t(warp * 32) << 16);
+        // warp w reads TMEM lane quarter w % 4, half w / 4 of the columns
+        const int quarter = warp & 3;
+        const int first = (warp >> 2) * (BN / 2);
+        const long long m = m0 + quarter * 32 + lane;
+        const uint32_t lane_base = tmem + (uint32_t(quarter * 32) << 16);
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
+        for (int c0 = first; c0 < first + BN / 2; c0 += 16) {
             float v[16];
             tmem_load16(lane_base + uint32_t(c0), v);
             epilogue16<BN, EPI>(g, m, int(n0) + c0, v, n_valid);
@@ -784,19 +819,29 @@ __global__ void begin_step(long long* step, float* loss, long long base) {
     }
 }
 
-// MSE head backward: dy = 2 (y - t) / B; dZ = bf16(dy * w * gelu'(Z)); loss
-// accumulated into loss[step - base - 1] (block partial sums, atomics).
-__global__ void head_backward(const float* __restrict__ y, const float* __restrict__ t, int rows,
-                              const float* __restrict__ w, const float* __restrict__ z, int width,
-                              float* __restrict__ dy, __nv_bfloat16* __restrict__ dz,
-                              const long long* step, float* loss, long long base) {
+// The output head of a training step, one warp per row: y = h . w + b (as
+// head_forward sums it), dy = 2 (y - t) / B, dZ = bf16(dy * w * gelu'(Z));
+// loss accumulated into loss[step - base - 1] (block partial sums, atomics).
+__global__ void head_step(const __nv_bfloat16* __restrict__ h, const float* __restrict__ t, int rows,
+                          const float* __restrict__ w, const float* __restrict__ b,
+                          const float* __restrict__ z, int width, float* __restrict__ dy,
+                          __nv_bfloat16* __restrict__ dz, const long long* step, float* loss,
+                          long long base) {
     __shared__ float part[8];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int r = blockIdx.x * (blockDim.x >> 5) + wib;
     float sq = 0.0f;
     if (r < rows) {
-        const float res = y[r] - t[r];
+        float acc = 0.0f;
+        for (int i = lane; i < width; i += 32) {
+            acc += __bfloat162float(h[(long long)r * width + i]) * w[i];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        }
+        const float res = acc + b[0] - t[r];
         const float d = 2.0f * res / float(rows);
         sq = res * res;
         if (lane == 0) {
@@ -857,16 +902,39 @@ __global__ void column_sums(const T* __restrict__ x, int rows, int cols, long lo
     }
 }
 
-// out[i] = sum over s < splits of partial[s * count + i], in split order.
-__global__ void sum_splits(const float* __restrict__ partial, int splits, long long count,
-                           float* __restrict__ out) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
-         i += (long long)gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int k = 0; k < splits; ++k) {
-            s += partial[k * count + i];
+// The gradient of a range of the flat parameter vector as partial products:
+// g[i] = sum over s < splits of partial[s * count + i - first], in split order.
+struct GradRange {
+    long long first, count;
+    const float* partial;
+    int splits;
+};
+constexpr int kMaxRanges = 14;      // weights and biases of at most 6 hidden layers and the head
+
+struct Gradient {
+    GradRange range[kMaxRanges];    // in parameter order, covering every parameter
+    int ranges;
+    __device__ __forceinline__ float at(long long i) const {
+        int k = 0;
+        while (k + 1 < ranges && i >= range[k + 1].first) {
+            ++k;
         }
-        out[i] = s;
+        const GradRange& r = range[k];
+        const float* p = r.partial + (i - r.first);
+        float s = 0.0f;
+        for (int j = 0; j < r.splits; ++j) {
+            s += p[j * r.count];
+        }
+        return s;
+    }
+};
+
+// The whole gradient written out (als_mlp_gradients; a training step adds the
+// partial products where Adam uses them).
+__global__ void write_gradient(Gradient g, long long n, float* __restrict__ out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
+        out[i] = g.at(i);
     }
 }
 
@@ -880,7 +948,7 @@ struct Segment {
 
 struct AdamArgs {
     float* p;
-    const float* g;
+    Gradient g;
     float* m;
     float* v;
     long long n;
@@ -896,7 +964,7 @@ __global__ void adam_update(AdamArgs a) {
     const float c2 = 1.0f - powf(a.beta2, float(t));
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n;
          i += (long long)gridDim.x * blockDim.x) {
-        const float gi = a.g[i];
+        const float gi = a.g.at(i);
         const float mi = a.beta1 * a.m[i] + (1.0f - a.beta1) * gi;
         const float vi = a.beta2 * a.v[i] + (1.0f - a.beta2) * gi * gi;
         a.m[i] = mi;

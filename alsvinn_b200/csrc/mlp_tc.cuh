@@ -1,6 +1,6 @@
 // BF16 tensor-core GEMM tile for the MLP surrogate (sm_100a, tcgen05).
 //
-// One CTA of 128 threads computes a 128 x BN tile of D = A * B^T, where
+// One CTA of 256 threads computes a 128 x BN tile of D = A * B^T, where
 // A is M x K and B is N x K (both read as "K-major" rows of K elements),
 // accumulating in FP32 in tensor memory (TMEM).  Operands go from global
 // memory through registers into shared memory in the canonical no-swizzle
@@ -11,9 +11,11 @@
 // 1024 bytes.  Strided staging lets the same kernel read transposed
 // operands (dZ^T, H^T, W^T) for the backward pass without extra copies.
 //
-// Two shared-memory stages: while the tensor core works on chunk c, the
-// threads stage chunk c+1; an mbarrier per stage, arrived on by
-// tcgen05.commit, says when a stage may be refilled.  Every wait is
+// gemm_stages<BN> shared-memory stages: with K no longer than that (every
+// training GEMM) all chunks are staged before the first MMA, so a tile waits
+// for memory once; otherwise the threads stage chunk c+1 while the tensor core
+// works on chunk c, and an mbarrier per stage, arrived on by tcgen05.commit,
+// says when a stage may be refilled.  Every wait is
 // bounded: on timeout the kernel records an error code, waits once more
 // (bounded) for its own MMAs, frees its TMEM and returns.
 #pragma once
@@ -25,7 +27,7 @@ namespace mlpk {
 
 constexpr int kTileM = 128;
 constexpr int kChunkK = 64;
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;
 constexpr unsigned kWaitLimit = 1u << 22;   // try_wait polls before giving up
 
 enum Epilogue {
@@ -255,7 +257,14 @@ __device__ __forceinline__ uint32_t staged_offset(int r, int kc) {
     return uint32_t((r >> 3) * 1024 + kc * 128 + (r & 7) * 16);
 }
 
-// Stages rows [row0, row0+ROWS) x K [k0, k0+64) of an operand into `dst`.
+// This thread's staging copies have landed and are visible to the tensor core.
+__device__ __forceinline__ void stage_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_async_shared();
+}
+
+// Stages rows [row0, row0+ROWS) x K [k0, k0+64) of an operand into `dst`;
+// 16-byte aligned rows when K is contiguous.
 template <int ROWS>
 __device__ __forceinline__ void stage_operand(unsigned char* dst, const Operand& op, long long row0,
                                               int k0) {
@@ -264,8 +273,11 @@ __device__ __forceinline__ void stage_operand(unsigned char* dst, const Operand&
         for (int idx = threadIdx.x; idx < ROWS * 8; idx += kThreads) {
             const int r = idx >> 3;
             const int kc = idx & 7;
-            const uint4 v = *reinterpret_cast<const uint4*>(op.p + (row0 + r) * op.rs + k0 + kc * 8);
-            *reinterpret_cast<uint4*>(dst + staged_offset(r, kc)) = v;
+            // asynchronous: complete after stage_wait
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                         ::"r"(smem_u32(dst + staged_offset(r, kc))),
+                           "l"(op.p + (row0 + r) * op.rs + k0 + kc * 8)
+                         : "memory");
         }
     } else {
         // transposed operand: consecutive rows are contiguous in memory
