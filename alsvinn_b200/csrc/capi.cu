@@ -98,7 +98,7 @@ int tile_extent(int precision, int dim, int d, int shape = 0) {
     return tile[d];
 }
 
-// Geometry of a padded grid and the tiles (of shape `shape`) covering the
+// Geometry of a padded grid and the tiles (of kernel `shape`) covering the
 // region [lo, hi).
 als::GridDesc make_grid(int dim, const int* n, int g, const int* lo, const int* hi,
     int precision = ALS_FP64, int shape = 0) {
@@ -113,6 +113,110 @@ als::GridDesc make_grid(int dim, const int* n, int g, const int* lo, const int* 
     }
     gd.plane = (long long)gd.N[0] * gd.N[1] * gd.N[2];
     gd.ghosts = g;
+    return gd;
+}
+
+// Rows per run of the 2-D warps that march along y, for a launch of
+// `strip_rows` rows of 32 cells in all.  A run costs about two rows besides
+// its own (the states outside it), so long runs are cheap; but a launch ends
+// with its last round of resident warps (148 SMs x rows_warps_per_sm), half
+// empty on average, so short runs waste less there.  With W rows per warp
+// slot and runs of r the loss is 2 / r + r / (2 W), least at r = 2 sqrt(W),
+// taken to the nearest split into whole rounds.  KH 1024^2 (W = 13.8), FP64,
+// ms per RK3 step: runs of 4 rows 0.268, 6 0.257, 8 0.240, 14 0.253, 16 0.279,
+// 32 0.475.
+int run_rows(long long strip_rows, int precision) {
+    const long long slots = 148LL *
+        (precision == ALS_FP64 ? als::rows_warps_per_sm<double>() : als::rows_warps_per_sm<float>());
+    const double w = double(strip_rows) / double(slots);
+    const double rounds = std::max(1.0, std::floor(0.5 * std::sqrt(w) + 0.5));
+    const double rows = std::ceil(w / rounds);
+    return int(std::min(double(als::kRunRows), std::max(2.0, rows)));
+}
+
+// Planes per segment of the 3-D blocks that march along z, for a launch of
+// `column_planes` planes of 16 x 16 cells in all: as run_rows, with about one
+// plane lost per segment and two resident blocks per SM.  FP64, ms: KH 128^3 x 2,
+// 4 steps, segments of 32 planes 8.29, 12 7.64, 8 7.50, 5 7.80, 2 9.11; 64^3, 16
+// steps, 16 planes 7.45, 8 4.35, 4 2.62, 2 2.92.
+int segment_planes(long long column_planes) {
+    const double w = double(column_planes) / (148.0 * ALS_ZMARCH_BLOCKS);
+    const double rounds = std::max(1.0, std::floor(std::sqrt(0.5 * w) + 0.5));
+    const double planes = std::ceil(w / rounds);
+    return int(std::min(double(ALS_ZMARCH_SEG), std::max(2.0, planes)));
+}
+
+long long strip_rows(const als::GridDesc& gd) {
+    return (long long)((gd.hi[0] - gd.lo[0] + als::kRunColumns - 1) / als::kRunColumns) *
+        (gd.hi[1] - gd.lo[1]);
+}
+
+// Splits the rows of a grid into runs of at most `rows`.
+void split_runs(als::GridDesc& gd, int rows) {
+    gd.tiles[1] = std::max(1, (gd.hi[1] - gd.lo[1] + rows - 1) / rows);
+}
+
+long long column_planes(const als::GridDesc& gd) {
+    return (long long)gd.tiles[0] * gd.tiles[1] * (gd.hi[2] - gd.lo[2]);
+}
+
+// Splits the planes of a grid into segments of at most `planes`.
+void split_segments(als::GridDesc& gd, int planes) {
+    gd.tiles[2] = std::max(1, (gd.hi[2] - gd.lo[2] + planes - 1) / planes);
+}
+
+long long region_cells(const als::GridDesc& gd) {
+    return (long long)(gd.hi[0] - gd.lo[0]) * (gd.hi[1] - gd.lo[1]) * (gd.hi[2] - gd.lo[2]);
+}
+
+// Kernel for levels of tile shape `shape` with `cells` cells in all.  A thread
+// per face has the least latency but repeats work at its boxes' edges, so it
+// runs 1-D and the smallest grids; warps that march along y do the least work
+// but need long runs, so they run the largest; in 2-D the 16 x 16 tiles lie
+// between.  16 RK3 steps, WENO2 + HLL3, ms, thread per face / 16 x 16 tiles /
+// marching: FP64 192^2 0.51 / 0.62 / 0.85, 256^2 0.61 / 0.67 / 0.92, 288^2 0.77 /
+// 0.69 / 0.95, 512^2 2.01 / 1.27 / 1.40, 576^2 2.51 / 1.55 / 1.63; FP32 256^2
+// 0.40 / 0.48 / 0.64, 288^2 0.56 / 0.51 / 0.68, 512^2 1.41 / 0.87 / 0.88, 576^2
+// 1.75 / 1.04 / 0.90 (MC and ENO3 cross in the same places).  3-D, thread per
+// face / marching along z: FP64 32^3 1.00 / 1.42, 40^3 1.53 / 1.53, 48^3 2.33 /
+// 1.56; FP32 32^3 0.76 / 0.93, 48^3 1.74 / 0.99.
+constexpr long long kFacesCells2 = 72000;
+constexpr long long kTilesCells2[2] = {400000, 270000};   // FP64, FP32
+constexpr long long kFacesCells3 = 60000;
+int choose_kernel(int dim, int flux, int shape, long long cells, int precision) {
+    if (als::stencil_flux(flux) || (dim == 2 && shape != 0)) {
+        return shape;
+    }
+    if (dim == 1 || cells <= (dim == 2 ? kFacesCells2 : kFacesCells3)) {
+        return als::kFacesKernel;
+    }
+    if (dim == 2 && als::kernel_built(2, 0, flux, 1) &&
+        cells <= kTilesCells2[precision == ALS_FP64 ? 0 : 1]) {
+        return 1;
+    }
+    return shape;
+}
+
+// The tile shape a configuration starts on: in 3-D the columns marching along
+// z where they are built (KH 128^3: faster than the boxes).
+int default_shape(int dim, int recon, int flux) {
+    return dim == 3 && als::shape_built(3, recon, flux, 1) ? 1 : 0;
+}
+
+// The grid, tiles and kernel of an FP64 flux evaluation over the region
+// [lo, hi) of `members` states.
+als::GridDesc plan_region(int dim, const int* n, int g, const int* lo, const int* hi, int recon,
+    int flux, int members, int* kernel) {
+    als::GridDesc gd = make_grid(dim, n, g, lo, hi);
+    *kernel = choose_kernel(dim, flux, default_shape(dim, recon, flux), region_cells(gd) * members,
+        ALS_FP64);
+    gd = make_grid(dim, n, g, lo, hi, ALS_FP64, *kernel);
+    if (als::marches_rows(dim, flux, *kernel)) {
+        split_runs(gd, run_rows(strip_rows(gd) * members, ALS_FP64));
+    }
+    if (als::marches_planes(dim, *kernel)) {
+        split_segments(gd, segment_planes(column_planes(gd) * members));
+    }
     return gd;
 }
 
@@ -259,6 +363,7 @@ cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t stream) {
 cudaError_t scratch_free(void* ptr, cudaStream_t stream) {
     return cudaFreeAsync(ptr, stream);
 }
+
 } // namespace als
 
 extern "C" {
@@ -424,7 +529,9 @@ int als_compute_flux(const als_grid* grid, int flux, int reconstruction, const d
     cudaStream_t s = (cudaStream_t)stream;
     als::StageParams P;
     std::memset(&P, 0, sizeof(P));
-    als::GridDesc gd = make_grid(grid->dimension, grid->n, grid->ghosts, lo, hi);
+    int kernel = 0;
+    als::GridDesc gd = plan_region(grid->dimension, grid->n, grid->ghosts, lo, hi,
+        reconstruction, flux, 1, &kernel);
     P.level[0] = plane_level(gd, nvar, (const void* const*)in, (const void* const*)in,
         (void* const*)out);
     P.nlevels = 1;
@@ -446,7 +553,8 @@ int als_compute_flux(const als_grid* grid, int flux, int reconstruction, const d
     if (!P.level[0].ws_out) {
         return fail(ALS_E_CUDA, "wave-speed scratch unavailable");
     }
-    ALS_CUDA(launch_stage(ALS_FP64, grid->dimension, reconstruction, flux, als::KIND_FLUX0, P, 0, s));
+    ALS_CUDA(launch_stage(ALS_FP64, grid->dimension, reconstruction, flux, als::KIND_FLUX0, P, 0, s,
+        kernel));
     if (!wave_speed) {
         return ALS_OK;
     }
@@ -586,7 +694,8 @@ namespace {
 struct SolverLevel {
     als_solver_config cfg;        // this level's n, lower, upper, members
     als::GridDesc grid;           // tiles of this level's tile shape
-    int shape = 0;                // tile shape of its stage kernels (stage_kernel.cuh)
+    int shape = 0;                // its tile shape (stage_kernel.cuh)
+    int kernel = 0;               // the kernel that runs its stages (plan_levels)
     int first = 0;                // global index of its first member
     long long member_elems = 0;   // nvar * plane
     double dx[3];
@@ -686,16 +795,16 @@ als::LevelDesc solver_level(const als_solver* s, const SolverLevel& L, const voi
     return D;
 }
 
-// Parameters of one stage over the levels of tile shape `shape`, in the
+// Parameters of one stage over the levels that kernel `kernel` runs, in the
 // solver's level order; `pick` chooses (in, un, out) per level.
 template<class Pick>
-als::StageParams solver_params(const als_solver* s, Pick pick, int shape = 0) {
+als::StageParams solver_params(const als_solver* s, Pick pick, int kernel) {
     als::StageParams P;
     std::memset(&P, 0, sizeof(P));
     P.nlevels = 0;
     for (size_t k = 0; k < s->levels.size(); ++k) {
         const SolverLevel& L = s->levels[s->order[k]];
-        if (L.shape != shape) {
+        if (L.kernel != kernel) {
             continue;
         }
         const void* in;
@@ -707,6 +816,7 @@ als::StageParams solver_params(const als_solver* s, Pick pick, int shape = 0) {
     P.bc = s->cfg.boundary;
     P.write_ghosts = 1;
     P.gamma = s->cfg.gamma;
+    P.chained = 1;
     P.counter = s->blocks_per_sm > 0 ? s->counter : nullptr;
     finish_params(P);
     return P;
@@ -722,20 +832,20 @@ cudaError_t launch_fe_update(als_solver* s, const SolverLevel& L) {
 }
 
 // Enqueues one time step of every level, each stage as one launch over all
-// levels of one tile shape (levels of different shapes take one launch per
-// shape, in shape order).  FE: FLUX0 + fe_update.  RK2: FLUX0 + RK2_1 into
+// levels of one kernel (levels of different tile shapes take one launch
+// each, in order).  FE: FLUX0 + fe_update.  RK2: FLUX0 + RK2_1 into
 // the other buffer (ping-pong).  RK3: FLUX0 + RK3_1 + RK3_2 in place.  With
 // `ev` (stages+1 events), records ev[0] before the first kernel and ev[k]
 // after the launches of stage k.
 template<class Pick>
 cudaError_t launch_stage_all(const als_solver* s, int kind, Pick pick) {
-    for (int shape = 0; shape < als::kMaxShapes; ++shape) {
-        als::StageParams P = solver_params(s, pick, shape);
+    for (int kernel = 0; kernel < als::kMaxKernels; ++kernel) {
+        als::StageParams P = solver_params(s, pick, kernel);
         if (P.nlevels == 0) {
             continue;
         }
         cudaError_t err = launch_stage(s->cfg.precision, s->cfg.dimension, s->cfg.reconstruction,
-            s->cfg.flux, kind, P, s->blocks_per_sm, s->stream, shape);
+            s->cfg.flux, kind, P, s->blocks_per_sm, s->stream, kernel);
         if (err != cudaSuccess) {
             return err;
         }
@@ -866,16 +976,43 @@ bool shape_available(const als_solver* s, int shape) {
         als::shape_built(s->cfg.dimension, s->cfg.reconstruction, s->cfg.flux, shape);
 }
 
+// Kernel and tiles of every level.  Levels of one tile shape share launches,
+// so their cells and rows count together.
+void plan_levels(als_solver* s) {
+    const int dim = s->cfg.dimension;
+    int lo[3] = {0, 0, 0};
+    for (SolverLevel& L : s->levels) {
+        long long cells = 0;
+        for (const SolverLevel& M : s->levels) {
+            cells += M.shape == L.shape ? region_cells(M.grid) * M.cfg.members : 0;
+        }
+        L.kernel = choose_kernel(dim, s->cfg.flux, L.shape, cells, s->cfg.precision);
+        L.grid = make_grid(dim, L.grid.n, s->g, lo, L.grid.n, s->cfg.precision, L.kernel);
+    }
+    long long rows = 0, planes = 0;
+    for (const SolverLevel& L : s->levels) {
+        if (als::marches_rows(dim, s->cfg.flux, L.kernel)) {
+            rows += strip_rows(L.grid) * L.cfg.members;
+        } else if (als::marches_planes(dim, L.kernel)) {
+            planes += column_planes(L.grid) * L.cfg.members;
+        }
+    }
+    for (SolverLevel& L : s->levels) {
+        if (als::marches_rows(dim, s->cfg.flux, L.kernel)) {
+            split_runs(L.grid, run_rows(rows, s->cfg.precision));
+        } else if (als::marches_planes(dim, L.kernel)) {
+            split_segments(L.grid, segment_planes(planes));
+        }
+    }
+}
+
 // Gives level l tile shape shapes[l] (available shapes only) and recovers
 // its tiles; the captured step graph no longer matches.
 void set_level_shapes(als_solver* s, const int* shapes) {
     for (size_t l = 0; l < s->levels.size(); ++l) {
-        SolverLevel& L = s->levels[l];
-        L.shape = shapes[l];
-        int lo[3] = {0, 0, 0};
-        L.grid = make_grid(s->cfg.dimension, L.grid.n, s->g, lo, L.grid.n, s->cfg.precision,
-            L.shape);
+        s->levels[l].shape = shapes[l];
     }
+    plan_levels(s);
     drop_graph(s);
 }
 
@@ -965,10 +1102,8 @@ int als_solver_create_levels(const als_solver_config* cfgs, int nlevels, int dev
         for (int d = 0; d < 3; ++d) {
             n[d] = d < cfg.dimension ? cfgs[l].n[d] : 1;
         }
-        // 3-D levels start on the z-marching columns where they are built
-        // (measured faster than the boxes on KH 128^3); the tuner may change it
-        L.shape = cfg.dimension == 3 &&
-            als::shape_built(3, cfg.reconstruction, cfg.flux, 1) ? 1 : 0;
+        // the tuner may change it
+        L.shape = default_shape(cfg.dimension, cfg.reconstruction, cfg.flux);
         L.grid = make_grid(cfg.dimension, n, s->g, lo, n, cfg.precision, L.shape);
         L.member_elems = (long long)s->nv * L.grid.plane;
         L.first = first;
@@ -990,6 +1125,7 @@ int als_solver_create_levels(const als_solver_config* cfgs, int nlevels, int dev
         }
         s->levels.push_back(L);
     }
+    plan_levels(s.get());
     s->members = first;
     s->order.resize(nlevels);
     std::iota(s->order.begin(), s->order.end(), 0);
@@ -1979,7 +2115,9 @@ extern "C" int als_compute_flux_static(const als_grid* grid, int flux, int recon
     const int nvar = grid->dimension + 2;
     als::StageParams P;
     std::memset(&P, 0, sizeof(P));
-    als::GridDesc gd = make_grid(grid->dimension, n, grid->ghosts, lo, n);
+    int kernel = 0;
+    als::GridDesc gd = plan_region(grid->dimension, n, grid->ghosts, lo, n,
+        reconstruction, flux, members, &kernel);
     const void* planes_in[als::kMaxVars];
     void* planes_out[als::kMaxVars];
     for (int v = 0; v < nvar; ++v) {
@@ -1999,7 +2137,7 @@ extern "C" int als_compute_flux_static(const als_grid* grid, int flux, int recon
     const size_t bytes = sizeof(unsigned long long) * 3 * size_t(members);
     ALS_CUDA(cudaMemsetAsync(scratch, 0, bytes, s));
     ALS_CUDA(launch_stage(ALS_FP64, grid->dimension, reconstruction, flux, als::KIND_FLUX0, P,
-        0, s));
+        0, s, kernel));
     // a non-negative double and its bit pattern read as an unsigned integer
     // are the same 8 bytes, so the maxima are copied straight into doubles
     ALS_CUDA(cudaMemcpyAsync(wave_speed, scratch, bytes, cudaMemcpyDeviceToHost, s));

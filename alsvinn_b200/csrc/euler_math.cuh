@@ -432,12 +432,10 @@ static __device__ __noinline__ double4 weno2_weights_plain(double d0, double d1)
     return w;
 }
 
-// d0, d1 >= 3e-16 by construction; below 2^400 every intermediate is normal.
-__device__ __forceinline__ double4 weno2_weights(double d0, double d1) {
-    const unsigned top = max(unsigned(__double2hiint(d0)), unsigned(__double2hiint(d1)));
-    if (top >= unsigned(hi_pow2(400))) {
-        return weno2_weights_plain(d0, d1);
-    }
+// The same by the straight-line division; d0, d1 >= 3e-16 by construction,
+// and below 2^400 (`ok`) every intermediate is normal.
+__device__ __forceinline__ double4 weno2_weights_quick(double d0, double d1, bool& ok) {
+    ok = max(unsigned(__double2hiint(d0)), unsigned(__double2hiint(d1))) < unsigned(hi_pow2(400));
     const double a0Left = rcp64(d0);
     const double a1Right = rcp64(d1);
     const double a1Left = 2.0 * a1Right;
@@ -451,6 +449,17 @@ __device__ __forceinline__ double4 weno2_weights(double d0, double d1) {
     w.y = quot64(a1Left, sl, yl);
     w.z = quot64(a0Right, sr, yr);
     w.w = quot64(a1Right, sr, yr);
+    return w;
+}
+
+// With DEFER the caller looks at `ok` and calls again without it when it is
+// false, so that its own code stays free of branches.
+template<bool DEFER>
+__device__ __forceinline__ double4 weno2_weights(double d0, double d1, bool& ok) {
+    double4 w = weno2_weights_quick(d0, d1, ok);
+    if (!DEFER && !ok) {
+        w = weno2_weights_plain(d0, d1);
+    }
     return w;
 }
 
@@ -540,8 +549,11 @@ __device__ __forceinline__ void wenof2_side(R w0, R w1, R gamma, const R* rho, c
     out[NSD + 1] = pp / (gamma - R(1)) + R(0.5) * pr * dot;
 }
 
-template<class R, int NV, int RECON, class Fetch>
-__device__ __forceinline__ void reconstruct_f(const Fetch& f, R* left, R* right, R gamma) {
+// DEFER (FP64 WENO2 and WENOF2): `ok` false asks for a call without it.
+template<class R, int NV, int RECON, bool DEFER, class Fetch>
+__device__ __forceinline__ void reconstruct_d(const Fetch& f, R* left, R* right, R gamma,
+    bool& ok) {
+    ok = true;
     if (RECON == RECON_NONE) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -569,7 +581,7 @@ __device__ __forceinline__ void reconstruct_f(const Fetch& f, R* left, R* right,
             w0Right = R(2) * d1 * rr;
             w1Right = d0 * rr;
         } else {
-            const double4 w = weno2_weights(d0, d1);
+            const double4 w = weno2_weights<DEFER>(d0, d1, ok);
             w0Left = w.x;
             w1Left = w.y;
             w0Right = w.z;
@@ -661,7 +673,7 @@ __device__ __forceinline__ void reconstruct_f(const Fetch& f, R* left, R* right,
             w0Right = R(2) * d1 * rr;
             w1Right = d0 * rr;
         } else {
-            const double4 w = weno2_weights(d0, d1);
+            const double4 w = weno2_weights<DEFER>(d0, d1, ok);
             w0Left = w.x;
             w1Left = w.y;
             w0Right = w.z;
@@ -724,6 +736,12 @@ __device__ __forceinline__ void reconstruct_f(const Fetch& f, R* left, R* right,
             right[v] = rv;
         }
     }
+}
+
+template<class R, int NV, int RECON, class Fetch>
+__device__ __forceinline__ void reconstruct_f(const Fetch& f, R* left, R* right, R gamma) {
+    bool ok;
+    reconstruct_d<R, NV, RECON, false>(f, left, right, gamma, ok);
 }
 
 // Stencil values from memory: variable v of the cell at `src` is v*vstride

@@ -6,7 +6,9 @@
 
 #include <cuda_runtime.h>
 
+#include "stage_faces.cuh"
 #include "stage_kernel.cuh"
+#include "stage_rows.cuh"
 #include "stage_zmarch.cuh"
 
 namespace als {
@@ -15,44 +17,30 @@ namespace als {
 // persistent launch of as many blocks as can be resident at once (or
 // `blocks_per_sm` per SM when > 0, capped by what fits), never more than
 // there are work items.
-// The kernel, block size and shared memory of one (shape, kind): the tiled
-// stage_kernel, or for 3-D shape 1 the z-marching kernel.
-template<class R, int DIM, int RECON, int FLUX, int KIND, int SHAPE>
-struct StageLaunch {
-    typedef StageLayout<R, DIM, RECON, FLUX, SHAPE> Lay;
-    static constexpr int THREADS = Lay::THREADS;
-    static constexpr size_t SMEM = Lay::SMEM;
-    static decltype(&stage_kernel<R, DIM, RECON, FLUX, KIND, SHAPE>) kernel() {
-        return stage_kernel<R, DIM, RECON, FLUX, KIND, SHAPE>;
-    }
-};
-template<class R, int RECON, int FLUX, int KIND>
-struct StageLaunch<R, 3, RECON, FLUX, KIND, 1> {
-    typedef ZLayout<R, RECON, FLUX> Lay;
-    static constexpr int THREADS = Lay::THREADS;
-    static constexpr size_t SMEM = Lay::SMEM;
-    static decltype(&zmarch_kernel<R, RECON, FLUX, KIND>) kernel() {
-        return zmarch_kernel<R, RECON, FLUX, KIND>;
-    }
-};
-
-template<class R, int DIM, int RECON, int FLUX, int KIND, int SHAPE>
-cudaError_t launch_stage_one(const StageParams& P, int blocks_per_sm, cudaStream_t stream) {
-    typedef StageLaunch<R, DIM, RECON, FLUX, KIND, SHAPE> Lay;
-    auto kernel = Lay::kernel();
+inline cudaError_t launch_stage_blocks(void (*kernel)(StageParams), int threads, size_t smem,
+    const StageParams& P, int blocks_per_sm, cudaStream_t stream) {
     // raising the dynamic shared-memory limit is idempotent and cheap; it is
     // done on every launch so that every device the process uses is covered
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        int(Lay::SMEM));
+        int(smem));
     if (err != cudaSuccess) {
         return err;
     }
     if (P.total_work <= 0) {
         return cudaSuccess;
     }
+    cudaLaunchAttribute chained;
+    chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    chained.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(unsigned(P.total_work));
+    config.blockDim = dim3(unsigned(threads));
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &chained;
+    config.numAttrs = P.chained ? 1 : 0;
     if (!P.counter) {
-        kernel<<<unsigned(P.total_work), Lay::THREADS, Lay::SMEM, stream>>>(P);
-        return cudaGetLastError();
+        return cudaLaunchKernelEx(&config, kernel, P);
     }
     int device = 0, sms = 0, resident = 0;
     err = cudaGetDevice(&device);
@@ -60,7 +48,7 @@ cudaError_t launch_stage_one(const StageParams& P, int blocks_per_sm, cudaStream
         err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     }
     if (err == cudaSuccess) {
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, Lay::THREADS, Lay::SMEM);
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
     }
     if (err != cudaSuccess) {
         return err;
@@ -75,8 +63,33 @@ cudaError_t launch_stage_one(const StageParams& P, int blocks_per_sm, cudaStream
     if (blocks > P.total_work) {
         blocks = P.total_work;
     }
-    kernel<<<unsigned(blocks), Lay::THREADS, Lay::SMEM, stream>>>(P);
-    return cudaGetLastError();
+    config.gridDim = dim3(unsigned(blocks));
+    return cudaLaunchKernelEx(&config, kernel, P);
+}
+
+// The kernel of one (kernel id, kind): a thread per face for id kFacesKernel
+// and for 1-D two-point fluxes; in 2-D id 0 with a two-point flux the warps
+// marching along y; in 3-D id 1 the columns marching along z; else the tiled
+// stage_kernel of that shape.
+template<class R, int DIM, int RECON, int FLUX, int KIND, int SHAPE>
+cudaError_t launch_stage_one(const StageParams& P, int b, cudaStream_t s) {
+    if constexpr (SHAPE == kFacesKernel) {
+        typedef FaceLayout<R, DIM, RECON, FLUX> Lay;
+        return launch_stage_blocks(faces_kernel<R, DIM, RECON, FLUX, KIND>, Lay::THREADS, Lay::SMEM,
+            P, b, s);
+    } else if constexpr (DIM == 3 && SHAPE == 1) {
+        typedef ZLayout<R, RECON, FLUX> Lay;
+        return launch_stage_blocks(zmarch_kernel<R, RECON, FLUX, KIND>, Lay::THREADS, Lay::SMEM, P,
+            b, s);
+    } else if constexpr (marches_rows(DIM, FLUX, SHAPE)) {
+        typedef RowLayout<R, RECON, FLUX> Lay;
+        // a block of the schedule stands for eight of these warps
+        return launch_stage_blocks(rows_kernel<R, RECON, FLUX, KIND>, 32, Lay::SMEM, P, 8 * b, s);
+    } else {
+        typedef StageLayout<R, DIM, RECON, FLUX, SHAPE> Lay;
+        return launch_stage_blocks(stage_kernel<R, DIM, RECON, FLUX, KIND, SHAPE>, Lay::THREADS,
+            Lay::SMEM, P, b, s);
+    }
 }
 
 template<class R, int DIM, int RECON, int FLUX, int SHAPE>
@@ -90,15 +103,22 @@ cudaError_t launch_stage_kind(int kind, const StageParams& P, int b, cudaStream_
     }
 }
 
-// The tile shape is a run-time choice among the shapes built for the
-// combination (shape_built).
+// The kernel is a run-time choice among those built for the combination
+// (kernel_built).
 template<class R, int DIM, int RECON, int FLUX>
-cudaError_t launch_stage_shape(int shape, int kind, const StageParams& P, int b, cudaStream_t s) {
-    if (shape == 0) {
-        return launch_stage_kind<R, DIM, RECON, FLUX, 0>(kind, P, b, s);
+cudaError_t launch_stage_shape(int kernel, int kind, const StageParams& P, int b, cudaStream_t s) {
+    if constexpr (kernel_built(DIM, RECON, FLUX, kFacesKernel)) {
+        if (kernel == kFacesKernel) {
+            return launch_stage_kind<R, DIM, RECON, FLUX, kFacesKernel>(kind, P, b, s);
+        }
     }
-    if constexpr (shape_built(DIM, RECON, FLUX, 1)) {
-        if (shape == 1) {
+    if constexpr (kernel_built(DIM, RECON, FLUX, 0)) {
+        if (kernel == 0) {
+            return launch_stage_kind<R, DIM, RECON, FLUX, 0>(kind, P, b, s);
+        }
+    }
+    if constexpr (kernel_built(DIM, RECON, FLUX, 1)) {
+        if (kernel == 1) {
             return launch_stage_kind<R, DIM, RECON, FLUX, 1>(kind, P, b, s);
         }
     }
@@ -143,10 +163,16 @@ cudaError_t launch_stage_dim(int recon, int flux, int kind, int shape, const Sta
     }
 }
 
-// Tile extents of `shape` (0 0 0 when that shape is not built for the dimension).
+// Cells per work item of kernel `shape` (0 0 0 when it is not built for the
+// dimension; the runs of the marching rows are split further by the host).
 template<int DIM>
 void stage_tile_dim(int shape, int* tile) {
     tile[0] = tile[1] = tile[2] = 0;
+    if (shape == kFacesKernel) {
+        tile[0] = FaceBox<DIM>::X;
+        tile[1] = FaceBox<DIM>::Y;
+        tile[2] = FaceBox<DIM>::Z;
+    }
     if (shape == 0) {
         tile[0] = TileShape<DIM, 0>::X;
         tile[1] = TileShape<DIM, 0>::Y;

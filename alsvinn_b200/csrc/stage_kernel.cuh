@@ -57,6 +57,12 @@ namespace als {
 // threads per SM, with registers to spare and no spills (0.384 vs 0.376).
 // All of these are build-time knobs; the FP32 units build with three blocks
 // per SM.
+//
+// These figures predate the straight-line division (exact64.cuh), which takes
+// the first row to 0.279.  The two-point fluxes run shape 0 with other kernels
+// since: marching warps on large grids (stage_rows.cuh, 0.244), a thread per
+// face on small ones (stage_faces.cuh); the tiles remain for the stencil
+// fluxes and for shape 1.
 #ifndef ALS_TILE2_X
 #define ALS_TILE2_X 32
 #endif
@@ -69,7 +75,7 @@ namespace als {
 #ifndef ALS_STAGE2_BLOCKS
 #define ALS_STAGE2_BLOCKS 2
 #endif
-// SHAPE 0 is each dimension's default tile.  2-D also builds SHAPE 1, a
+// SHAPE 0 is the default tile in 1-D and 2-D.  2-D also builds SHAPE 1, a
 // 16 x 16 tile of 288 threads: more halo work per cell than 32 x 16, but
 // more resident blocks per SM and finer work items, which can pay on small
 // grids or many members; the schedule tuner chooses per grid level
@@ -149,6 +155,31 @@ __host__ __device__ constexpr bool shape_built(int dim, int recon, int flux, int
 }
 constexpr int kMaxShapes = 2;
 
+// The kernel that runs a level's stages: that of its tile shape, or
+// kFacesKernel, one thread per face (stage_faces.cuh).
+constexpr int kFacesKernel = 2;
+constexpr int kMaxKernels = 3;
+
+// Two-point fluxes have it in every dimension; in 1-D it is the only one.  In
+// 2-D the 16 x 16 tiles also serve levels of shape 0 (als_solver_set_tiles
+// offers shape 1 where shape_built says), so they are built for every
+// reconstruction.
+__host__ __device__ constexpr bool kernel_built(int dim, int recon, int flux, int kernel) {
+    return kernel == kFacesKernel ? !stencil_flux(flux)
+        : (dim == 2 && kernel == 1 && flux <= FLUX_CENTRAL) ||
+            (shape_built(dim, recon, flux, kernel) && (dim > 1 || stencil_flux(flux)));
+}
+
+// Whether a kernel's work items are runs of rows (stage_rows.cuh).
+__host__ __device__ constexpr bool marches_rows(int dim, int flux, int kernel) {
+    return dim == 2 && kernel == 0 && !stencil_flux(flux);
+}
+
+// Whether they are segments of planes (stage_zmarch.cuh).
+__host__ __device__ constexpr bool marches_planes(int dim, int kernel) {
+    return dim == 3 && kernel == 1;
+}
+
 template<class R, int DIM, int RECON, int FLUX, int SHAPE = 0>
 struct StageLayout {
     static constexpr int NV = DIM + 2;
@@ -186,18 +217,25 @@ struct StageLayout {
 
 // dt of the step (Integrator.cpp:20-46) followed by the end-time clamp
 // (FixedIntervalWriter.cpp:45-53): dt = min(cfl / sum_d ws_d/dx_d, T - t).
-__device__ __forceinline__ double step_dt(const StepState* st) {
+__device__ __forceinline__ double step_dt_of(const double* ws, const double* dx, double cfl,
+    double end_time, double t) {
     double total = 0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        if (st->dx[d] == 0) {
+        if (dx[d] == 0) {
             continue;
         }
-        total += __longlong_as_double((long long)st->ws[d]) / st->dx[d];
+        total += ws[d] / dx[d];
     }
-    double dt = st->cfl / total;
-    const double rest = st->end_time - st->t;
+    const double dt = cfl / total;
+    const double rest = end_time - t;
     return rest < dt ? rest : dt;
+}
+
+__device__ __forceinline__ double step_dt(const StepState* st) {
+    const double ws[3] = {__longlong_as_double((long long)st->ws[0]),
+        __longlong_as_double((long long)st->ws[1]), __longlong_as_double((long long)st->ws[2])};
+    return step_dt_of(ws, st->dx, st->cfl, st->end_time, st->t);
 }
 
 // Padded positions that hold a copy of interior cell i along one direction
@@ -476,51 +514,64 @@ __device__ __forceinline__ void finish_step(StepState* st) {
     }
 }
 
-// The stage combination of one updated cell (interior coordinates gx, gy,
-// gz; its net flux `acc`; `ub`, its value of the stage's input state as
-// staged) and its writes: the cell, its boundary images (or, for a split
-// grid, the neighbouring subdomains' ghost cells), and, after the last
-// stage, the constraint check.
+// The stage combination of one value: x its net flux, ub its value of the
+// stage's input state, un its U^n.
+template<class R, int KIND>
+__device__ __forceinline__ R combine_stage(R x, R c, R ub, R un) {
+    if (KIND == KIND_RK2_1) {
+        // RungeKutta2.cpp:57-63
+        x = x * c;
+        x = x + ub;
+        x = x + un;
+        x = x * R(0.5);
+    } else if (KIND == KIND_RK3_1) {
+        // RungeKutta3.cpp:65-78
+        x = x * c;
+        x = x + ub;
+        x = x * R(1. / 3.);
+        x = x + un;
+        x = x * R(3. / 4.);
+    } else if (KIND == KIND_RK3_2) {
+        // RungeKutta3.cpp:65-83
+        x = x * c;
+        x = x + ub;
+        x = x * R(2);
+        x = x + un;
+        x = x * R(1. / 3.);
+    }
+    return x;
+}
+
+// U^n of a cell of the region for update_cell (nothing for the flux stage).
 template<class R, int DIM, int NV, int KIND>
-__device__ __forceinline__ void update_cell(const StageParams& P, const LevelDesc& L, int member,
-    long long base, R c, R gamma, const R* acc, const R* ub, int gx, int gy, int gz, bool& bad,
+__device__ __forceinline__ void load_un(const LevelDesc& L, long long base, int gx, int gy, int gz,
+    R* un) {
+    if (KIND != KIND_FLUX0) {
+        const GridDesc& gd = L.grid;
+        const long long row = (long long)(DIM > 2 ? gz + gd.ghosts : 0) * gd.N[1] +
+            (DIM > 1 ? gy + gd.ghosts : 0);
+        const long long idx = row * gd.N[0] + gx + gd.ghosts;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            un[v] = (static_cast<const R*>(L.un[v]) + base)[idx];
+        }
+    }
+}
+
+// The writes of one updated cell (interior coordinates gx, gy, gz): the cell,
+// its boundary images (or, for a split grid, the neighbouring subdomains'
+// ghost cells), and, with `check` (after the last stage), the constraint check.
+template<class R, int DIM, int NV>
+__device__ __forceinline__ void write_cell(const StageParams& P, const LevelDesc& L, int member,
+    long long base, R gamma, const R* val, bool check, int gx, int gy, int gz, bool& bad,
     long long& bad_idx) {
-    constexpr bool LAST = KIND == KIND_RK3_2 || KIND == KIND_RK2_1;
     const GridDesc& gd = L.grid;
     const StepState* st = L.state ? L.state + (L.subdomains ? 0 : member) : nullptr;
-    auto unp = [&](int v) { return static_cast<const R*>(L.un[v]) + base; };
     auto outp = [&](int v) { return static_cast<R*>(L.out[v]) + base; };
     const int px = gx + gd.ghosts;
     const int py = DIM > 1 ? gy + gd.ghosts : 0;
     const int pz = DIM > 2 ? gz + gd.ghosts : 0;
     const long long idx = ((long long)pz * gd.N[1] + py) * gd.N[0] + px;
-    R val[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        R x = acc[v];
-        if (KIND == KIND_RK2_1) {
-            // RungeKutta2.cpp:57-63
-            x = x * c;
-            x = x + ub[v];
-            x = x + unp(v)[idx];
-            x = x * R(0.5);
-        } else if (KIND == KIND_RK3_1) {
-            // RungeKutta3.cpp:65-78
-            x = x * c;
-            x = x + ub[v];
-            x = x * R(1. / 3.);
-            x = x + unp(v)[idx];
-            x = x * R(3. / 4.);
-        } else if (KIND == KIND_RK3_2) {
-            // RungeKutta3.cpp:65-83
-            x = x * c;
-            x = x + ub[v];
-            x = x * R(2);
-            x = x + unp(v)[idx];
-            x = x * R(1. / 3.);
-        }
-        val[v] = x;
-    }
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         outp(v)[idx] = val[v];
@@ -583,11 +634,27 @@ __device__ __forceinline__ void update_cell(const StageParams& P, const LevelDes
             }
         }
     }
-    if (LAST && st && !obeys_constraints<R, NV>(val, gamma)) {
+    if (check && st && !obeys_constraints<R, NV>(val, gamma)) {
         bad = true;
         // subdomains: the member's padded plane offset first
         bad_idx = L.subdomains ? (long long)member * gd.plane + idx : idx;
     }
+}
+
+// The stage combination of one updated cell (its net flux `acc`; `ub`, its
+// value of the stage's input state as staged; `un`, its U^n, see load_un) and
+// its writes.
+template<class R, int DIM, int NV, int KIND>
+__device__ __forceinline__ void update_cell(const StageParams& P, const LevelDesc& L, int member,
+    long long base, R c, R gamma, const R* acc, const R* ub, const R* un, int gx, int gy, int gz,
+    bool& bad, long long& bad_idx) {
+    R val[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        val[v] = combine_stage<R, KIND>(acc[v], c, ub[v], un[v]);
+    }
+    write_cell<R, DIM, NV>(P, L, member, base, gamma, val, KIND == KIND_RK3_2 || KIND == KIND_RK2_1,
+        gx, gy, gz, bad, bad_idx);
 }
 
 // One work item: tile `tile` of member `member` of level L.
@@ -704,7 +771,9 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const LevelDesc
         for (int v = 0; v < NV; ++v) {
             ub[v] = box[v * Lay::BOX + bidx];
         }
-        update_cell<R, DIM, NV, KIND>(P, L, member, base, c, gamma, acc[k], ub, gx, gy, gz, bad,
+        R un[NV];
+        load_un<R, DIM, NV, KIND>(L, base, gx, gy, gz, un);
+        update_cell<R, DIM, NV, KIND>(P, L, member, base, c, gamma, acc[k], ub, un, gx, gy, gz, bad,
             bad_idx);
     }
 
@@ -748,48 +817,41 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const LevelDesc
     }
 }
 
-// Work item w of the launch: its level, member and tile, skipping members
-// that are done.
-template<class R, int DIM, int RECON, int FLUX, int SHAPE, int KIND>
-__device__ __forceinline__ void stage_item(const StageParams& P, long long w, unsigned char* smem) {
-    int l = 0;
-#pragma unroll
-    for (int k = 1; k < kMaxLevels; ++k) {
-        if (k < P.nlevels && w >= P.level[k].work_begin) {
-            l = k;
-        }
-    }
-    const LevelDesc& L = P.level[l];
-    const long long local = w - L.work_begin;
-    const int member = int(local / L.tiles_per_member);
-    const int tile = int(local - (long long)member * L.tiles_per_member);
-    if (L.state) {
-        const volatile StepState* st = L.state + (L.subdomains ? 0 : member);
-        if (st->done) {
-            return;
-        }
-    }
-    stage_tile<R, DIM, RECON, FLUX, SHAPE, KIND>(P, L, tile, member, smem);
-}
-
-// Two launch modes.  Without a work counter every block takes the work item
-// of its index (the hardware hands out blocks as SMs free up).  With one,
-// the launch is persistent: a fixed number of resident blocks take items
-// from the counter until the list is exhausted, and the last block to
-// leave resets the counter for the next launch.
-template<class R, int DIM, int RECON, int FLUX, int KIND, int SHAPE = 0>
-__global__ void __launch_bounds__((StageLayout<R, DIM, RECON, FLUX, SHAPE>::THREADS),
-    (StageLayout<R, DIM, RECON, FLUX, SHAPE>::BLOCKS))
-stage_kernel(const StageParams P) {
-    extern __shared__ __align__(16) unsigned char smem[];
+// The work items of this block, run(level, tile, member) for each, skipping
+// members that are done.  Two launch modes: without a work counter every
+// block takes the work item of its index (the hardware hands out blocks as
+// SMs free up); with one, the launch is persistent: a fixed number of
+// resident blocks take items from the counter until the list is exhausted,
+// and the last block to leave resets the counter for the next launch.
+template<class Tile>
+__device__ __forceinline__ void walk_work(const StageParams& P, Tile run) {
     __shared__ long long item;
+    // the solver's stages follow one another with programmatic launches: the
+    // next stage's blocks may take their places now and wait here for this
+    // one to finish (a no-op for other launches)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x == 0) {
         item = P.counter ? (long long)atomicAdd(&P.counter[0], 1ull) : (long long)blockIdx.x;
     }
     __syncthreads();
     // one call site, so the tile code is inlined once
     for (long long w = item; w < P.total_work;) {
-        stage_item<R, DIM, RECON, FLUX, SHAPE, KIND>(P, w, smem);
+        int l = 0;
+#pragma unroll
+        for (int k = 1; k < kMaxLevels; ++k) {
+            if (k < P.nlevels && w >= P.level[k].work_begin) {
+                l = k;
+            }
+        }
+        const LevelDesc& L = P.level[l];
+        const long long local = w - L.work_begin;
+        const int member = int(local / L.tiles_per_member);
+        const int tile = int(local - (long long)member * L.tiles_per_member);
+        const volatile StepState* st = L.state ? L.state + (L.subdomains ? 0 : member) : nullptr;
+        if (!st || !st->done) {
+            run(L, tile, member);
+        }
         if (!P.counter) {
             break;
         }
@@ -810,6 +872,16 @@ stage_kernel(const StageParams P) {
             __threadfence();
         }
     }
+}
+
+template<class R, int DIM, int RECON, int FLUX, int KIND, int SHAPE = 0>
+__global__ void __launch_bounds__((StageLayout<R, DIM, RECON, FLUX, SHAPE>::THREADS),
+    (StageLayout<R, DIM, RECON, FLUX, SHAPE>::BLOCKS))
+stage_kernel(const StageParams P) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    walk_work(P, [&](const LevelDesc& L, int tile, int member) {
+        stage_tile<R, DIM, RECON, FLUX, SHAPE, KIND>(P, L, tile, member, smem);
+    });
 }
 
 } // namespace als

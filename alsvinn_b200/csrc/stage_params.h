@@ -16,6 +16,9 @@ enum Boundary { BC_NEUMANN = 0, BC_PERIODIC = 1 };
 
 constexpr int kMaxVars = 5;
 constexpr int kMaxLevels = 4;
+// the warps marching along y (stage_rows.cuh): columns, and most rows, of a run
+constexpr int kRunColumns = 32;
+constexpr int kRunRows = 32;
 
 // Per-simulation time-stepping state kept on the device, so a whole time
 // step runs without a host round trip.  One per ensemble member.
@@ -41,7 +44,7 @@ struct alignas(64) StepState {
 struct GridDesc {
     int n[3];          // interior cells (1 for inactive directions)
     int N[3];          // padded extents
-    int tiles[3];      // tiles covering the region [lo, hi)
+    int tiles[3];      // tiles covering the region [lo, hi) (2-D marching warps: strips, runs)
     int lo[3], hi[3];  // region of interior cells to update (interior coordinates)
     long long plane;   // padded cells per plane
     int ghosts;        // ghost width of the planes (>= the stencil's)
@@ -80,6 +83,7 @@ struct StageParams {
     int write_ghosts;        // 1: also write the boundary images of every updated cell
     double gamma;
     double c_fixed;          // dt/dx for stages when a level has no state
+    int chained;             // 1: a stage of the solver, launched while the one before it finishes
     unsigned long long* counter; // persistent mode: [next item, blocks done], zero between launches; null: one item per block
 };
 

@@ -1,7 +1,7 @@
 // 3-D stage kernel that marches along z (tile shape 1 of the 3-D stage).
 //
-// A block owns a 16 x 16 column of cells over a segment of ALS_ZMARCH_SEG
-// cells along z.  It keeps a ring of three x-y planes (each with its x-y halo of
+// A block owns a 16 x 16 column of cells over a segment of at most
+// ALS_ZMARCH_SEG cells along z (the host chooses the length).  It keeps a ring of three x-y planes (each with its x-y halo of
 // G cells, every conserved variable) in shared memory and walks the segment
 // plane by plane.  Per plane, the x and y directions reconstruct and
 // evaluate their faces like the 2-D kernel; then the thread of each column
@@ -30,7 +30,6 @@ struct ZLayout {
     static constexpr int S = recon_ghosts(RECON) - 1;   // stencil half-width along z
     static constexpr int TX = Shape::X;
     static constexpr int TY = Shape::Y;
-    static constexpr int SEG = Shape::Z;
     static constexpr int BX = TX + 2 * G;
     static constexpr int BY = TY + 2 * G;
     static constexpr int PLANE = BX * BY;
@@ -169,8 +168,10 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
     const int tz = tile / (gd.tiles[0] * gd.tiles[1]);
     const int x0 = gd.lo[0] + tx * Lay::TX;
     const int y0 = gd.lo[1] + ty * Lay::TY;
-    const int k0 = gd.lo[2] + tz * Lay::SEG;
-    const int k1 = k0 + Lay::SEG < gd.hi[2] ? k0 + Lay::SEG : gd.hi[2];
+    // segment tz of gd.tiles[2], which split the planes evenly
+    const int nz = gd.hi[2] - gd.lo[2];
+    const int k0 = gd.lo[2] + int((long long)nz * tz / gd.tiles[2]);
+    const int k1 = gd.lo[2] + int((long long)nz * (tz + 1) / gd.tiles[2]);
     const long long base = (long long)member * L.member_stride;
     auto inp = [&](int v) { return static_cast<const R*>(L.in[v]) + base; };
     auto unp = [&](int v) { return static_cast<const R*>(L.un[v]) + base; };
@@ -310,7 +311,9 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
                 for (int v = 0; v < NV; ++v) {
                     ub[v] = pl[v * Lay::PLANE + coff];
                 }
-                update_cell<R, 3, NV, KIND>(P, L, member, base, c, gamma, acc, ub, x0 + cx, y0 + cy,
+                R un[NV];
+                load_un<R, 3, NV, KIND>(L, base, x0 + cx, y0 + cy, k, un);
+                update_cell<R, 3, NV, KIND>(P, L, member, base, c, gamma, acc, ub, un, x0 + cx, y0 + cy,
                     k, bad, bad_idx);
             }
         }
@@ -356,60 +359,13 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
 }
 
 template<class R, int RECON, int FLUX, int KIND>
-__device__ __forceinline__ void zmarch_item(const StageParams& P, long long w, unsigned char* smem) {
-    int l = 0;
-#pragma unroll
-    for (int k = 1; k < kMaxLevels; ++k) {
-        if (k < P.nlevels && w >= P.level[k].work_begin) {
-            l = k;
-        }
-    }
-    const LevelDesc& L = P.level[l];
-    const long long local = w - L.work_begin;
-    const int member = int(local / L.tiles_per_member);
-    const int tile = int(local - (long long)member * L.tiles_per_member);
-    if (L.state) {
-        const volatile StepState* st = L.state + (L.subdomains ? 0 : member);
-        if (st->done) {
-            return;
-        }
-    }
-    zmarch_tile<R, RECON, FLUX, KIND>(P, L, tile, member, smem);
-}
-
-// Launch modes as stage_kernel: one block per work item, or persistent
-// blocks taking items from the counter.
-template<class R, int RECON, int FLUX, int KIND>
 __global__ void __launch_bounds__((ZLayout<R, RECON, FLUX>::THREADS),
     (ZLayout<R, RECON, FLUX>::BLOCKS))
 zmarch_kernel(const StageParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ long long item;
-    if (threadIdx.x == 0) {
-        item = P.counter ? (long long)atomicAdd(&P.counter[0], 1ull) : (long long)blockIdx.x;
-    }
-    __syncthreads();
-    for (long long w = item; w < P.total_work;) {
-        zmarch_item<R, RECON, FLUX, KIND>(P, w, smem);
-        if (!P.counter) {
-            break;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            item = (long long)atomicAdd(&P.counter[0], 1ull);
-        }
-        __syncthreads();
-        w = item;
-    }
-    if (P.counter && threadIdx.x == 0) {
-        __threadfence();
-        const unsigned long long prev = atomicAdd(&P.counter[1], 1ull);
-        if (prev == gridDim.x - 1) {
-            P.counter[0] = 0;
-            P.counter[1] = 0;
-            __threadfence();
-        }
-    }
+    walk_work(P, [&](const LevelDesc& L, int tile, int member) {
+        zmarch_tile<R, RECON, FLUX, KIND>(P, L, tile, member, smem);
+    });
 }
 
 } // namespace als

@@ -1,0 +1,107 @@
+"""The stage kernels and the rules that choose between them, against the C
+oracle bit for bit, at the sizes where they can go wrong.
+
+2-D grids above 400,000 cells (FP64) march warps along y (runs of rows, strips
+of 32 columns), those below 72,000 and 3-D grids below 60,000 take a thread per
+face, 2-D grids between take 16 x 16 tiles, larger 3-D grids march blocks along z
+(segments of planes, 16 x 16 columns).
+"""
+import numpy as np
+import pytest
+
+from oracle_lib import ghost_cells, smooth_random_state
+
+torch = pytest.importorskip("torch")
+
+import alsvinn_b200 as als  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def _flux_case(c_oracle, dim, n, recon, flux, start=(0, 0, 0), end=(0, 0, 0)):
+    g = ghost_cells(recon, flux)
+    st = smooth_random_state(sum(n) + len(recon), dim, n, g)
+    cfg = c_oracle.config(dim, n, [0.0] * dim, [1.0] * dim, flux, recon, "rungekutta3", "periodic", 1.4)
+    st = c_oracle.fill_ghosts(cfg, st)
+    expect, ws = c_oracle.net_flux(cfg, st)
+    out = torch.full(st.shape, -7.0, dtype=torch.float64, device="cuda")
+    got_ws = als.NumericalFlux(dim, n, flux, recon).computeFlux(torch.from_numpy(st).cuda(), out,
+                                                                 start, end)
+    box = [slice(None)]
+    for d in (2, 1, 0):
+        box.append(slice(g + start[d], g + n[d] + end[d]) if d < dim else slice(None))
+    got = out.cpu().numpy()
+    np.testing.assert_array_equal(got[tuple(box)], expect[tuple(box)])
+    # nothing outside the region is written
+    got[tuple(box)] = -7.0
+    assert (got == -7.0).all()
+    return got_ws, ws
+
+
+LARGE = [(32, 12600), (12601, 33), (703, 631), (1023, 401), (1025, 399), (353, 331), (272, 265)]
+RECONS = ["none", "weno2", "eno2", "eno3", "eno4", "mc", "mm", "wenof2", "weno3"]
+
+
+@pytest.mark.parametrize("n", LARGE, ids=lambda n: "x".join(map(str, n)))
+@pytest.mark.parametrize("recon", ["weno2", "eno4"])
+def test_marching_rows_sizes(c_oracle, n, recon):
+    got, ws = _flux_case(c_oracle, 2, n, recon, "hll3")
+    np.testing.assert_array_equal(got[:2], ws[:2])
+
+
+@pytest.mark.parametrize("recon", RECONS)
+@pytest.mark.parametrize("flux", ["hll", "hll3", "central"])
+def test_marching_rows_schemes(c_oracle, recon, flux):
+    got, ws = _flux_case(c_oracle, 2, (801, 503), recon, flux)
+    np.testing.assert_array_equal(got[:2], ws[:2])
+
+
+@pytest.mark.parametrize("recon", RECONS)
+def test_tiles_schemes(c_oracle, recon):
+    got, ws = _flux_case(c_oracle, 2, (301, 263), recon, "hll3")
+    np.testing.assert_array_equal(got[:2], ws[:2])
+
+
+def test_marching_rows_regions(c_oracle):
+    _flux_case(c_oracle, 2, (811, 603), "weno2", "hll3", start=(3, 2, 0), end=(-5, -1, 0))
+    _flux_case(c_oracle, 2, (811, 703), "eno3", "hll", start=(0, 40, 0), end=(-70, 0, 0))
+
+
+@pytest.mark.parametrize("n", [(7, 9), (16, 7), (17, 8), (33, 64), (260, 252)],
+                         ids=lambda n: "x".join(map(str, n)))
+@pytest.mark.parametrize("recon", ["none", "weno2", "eno3", "weno3"])
+def test_faces_2d(c_oracle, n, recon):
+    got, ws = _flux_case(c_oracle, 2, n, recon, "hll3")
+    np.testing.assert_array_equal(got[:2], ws[:2])
+
+
+@pytest.mark.parametrize("n", [(8, 8, 8), (9, 5, 7), (17, 13, 10), (33, 40, 41), (40, 41, 42)],
+                         ids=lambda n: "x".join(map(str, n)))
+@pytest.mark.parametrize("recon", ["weno2", "mc"])
+def test_3d(c_oracle, n, recon):
+    got, ws = _flux_case(c_oracle, 3, n, recon, "hll3")
+    np.testing.assert_array_equal(got, ws)
+
+
+@pytest.mark.parametrize("n", [4, 5, 127, 128, 254, 1000], ids=str)
+@pytest.mark.parametrize("recon", ["none", "weno2"])
+def test_faces_1d(c_oracle, n, recon):
+    got, ws = _flux_case(c_oracle, 1, (n,), recon, "hll")
+    np.testing.assert_array_equal(got[:1], ws[:1])
+
+
+@pytest.mark.parametrize("dim,n", [(2, (700, 579)), (2, (400, 270)), (3, (33, 47, 41)), (3, (50, 16, 81))],
+                         ids=["700x579", "400x270", "33x47x41", "50x16x81"])
+@pytest.mark.parametrize("integ", ["rungekutta3", "rungekutta2", "forwardeuler"])
+@pytest.mark.parametrize("bc", ["periodic", "neumann"])
+def test_marching_steps(c_oracle, dim, n, integ, bc):
+    st = smooth_random_state(5 + dim, dim, n, 2)
+    cfg = c_oracle.config(dim, n, [0.0] * dim, [1.0] * dim, "hll3", "weno2", integ, bc, 1.4)
+    rc, expect, dts, steps, t = c_oracle.simulate(cfg, st, 0.4, 1.0, max_steps=3)
+    with als.Simulator(dim, n, flux="hll3", reconstruction="weno2", integrator=integ, boundary=bc,
+                       cfl=0.4, end_time=1.0, max_steps=3) as sim:
+        sim.set_state(st)
+        sim.run()
+        info = sim.info()
+        np.testing.assert_array_equal(sim.get_state()[0], expect)
+    assert info["steps"] == steps and info["t"] == t
