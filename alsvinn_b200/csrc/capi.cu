@@ -917,6 +917,59 @@ int enqueue_step(als_solver* s, cudaEvent_t* ev = nullptr) {
     return ALS_OK;
 }
 
+// Whether whole steps of this solver run in one launch (stage_line.cuh):
+// 1-D RK2 / RK3 with a two-point flux and lines that fit a cluster's shared
+// memory.
+bool runs_lines(const als_solver* s) {
+    if (s->cfg.dimension != 1 || s->subdomains || s->cfg.flux > ALS_FLUX_CENTRAL ||
+        (s->cfg.integrator != ALS_INT_RK2 && s->cfg.integrator != ALS_INT_RK3)) {
+        return false;
+    }
+    for (const SolverLevel& L : s->levels) {
+        if (L.grid.n[0] > als::kLineBlocks * als::kLineCells) {
+            return false;
+        }
+    }
+    return true;
+}
+
+// Enqueues `steps` time steps of every line, at most kLineSteps per launch
+// (about 5 us each).
+int enqueue_lines(als_solver* s, long long steps) {
+    const long long kLineSteps = 2048;
+    const bool rk3 = s->cfg.integrator == ALS_INT_RK3;
+    while (steps > 0) {
+        const int count = int(std::min(steps, kLineSteps));
+        for (const SolverLevel& L : s->levels) {
+            als::LineParams P;
+            std::memset(&P, 0, sizeof(P));
+            P.in = s->current(L);
+            P.even = s->current(L);
+            P.odd = rk3 ? s->current(L) : s->other(L);
+            P.state = s->state + L.first;
+            P.plane = L.grid.plane;
+            P.n = L.grid.n[0];
+            P.ghosts = s->g;
+            P.bc = s->cfg.boundary;
+            P.steps = count;
+            P.gamma = s->cfg.gamma;
+            // pieces of 64 cells or more, which also covers any stencil
+            int blocks = als::kLineBlocks;
+            while (blocks > 1 && P.n / blocks < 64) {
+                blocks /= 2;
+            }
+            P.stride = (P.n + blocks - 1) / blocks + 2 * s->g;
+            ALS_CUDA((s->cfg.precision == ALS_FP64 ? als::launch_line_f64 : als::launch_line_f32)(
+                s->cfg.reconstruction, s->cfg.flux, rk3, P, L.cfg.members, blocks, s->stream));
+        }
+        if (!rk3) {
+            s->cur ^= count & 1;
+        }
+        steps -= count;
+    }
+    return ALS_OK;
+}
+
 template<class R>
 int fill_member_ghosts(als_solver* s, const SolverLevel& L, void* base, int first_local,
     int count) {
@@ -1396,6 +1449,9 @@ int als_solver_advance(als_solver* s, long long steps) {
         return fail(ALS_E_INVALID, "set the state of the split grid after als_solver_decompose");
     }
     DeviceGuard guard(s->device);
+    if (runs_lines(s)) {
+        return enqueue_lines(s, steps);
+    }
     // whole time steps are captured once into a CUDA graph and replayed; the
     // RK2 ping-pong needs an even number of steps per graph
     const int per_graph = 8;

@@ -8,6 +8,7 @@
 
 #include "stage_faces.cuh"
 #include "stage_kernel.cuh"
+#include "stage_line.cuh"
 #include "stage_rows.cuh"
 #include "stage_zmarch.cuh"
 
@@ -163,6 +164,62 @@ cudaError_t launch_stage_dim(int recon, int flux, int kind, int shape, const Sta
     }
 }
 
+// Whole steps of `members` 1-D lines, one cluster of `blocks` blocks each.
+template<class R, int RECON, int FLUX, bool RK3>
+cudaError_t launch_line_one(const LineParams& P, int members, int blocks, cudaStream_t stream) {
+    auto kernel = line_kernel<R, RECON, FLUX, RK3>;
+    const size_t smem = LineLayout<R, RECON, FLUX>::smem(P.stride);
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        int(smem));
+    if (err != cudaSuccess) {
+        return err;
+    }
+    // a thread per face of the largest piece, up to kLineThreads
+    const int faces = P.stride - 2 * P.ghosts + 1;
+    const int threads = faces < kLineThreads ? (faces + 31) / 32 * 32 : kLineThreads;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = unsigned(blocks);
+    cluster.val.clusterDim.y = 1;
+    cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(unsigned(members) * unsigned(blocks));
+    config.blockDim = dim3(unsigned(threads));
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &cluster;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, P);
+}
+
+template<class R, int RECON>
+cudaError_t launch_line_flux(int flux, bool rk3, const LineParams& P, int members, int blocks,
+    cudaStream_t s) {
+    switch (flux) {
+    case FLUX_HLL: return rk3 ? launch_line_one<R, RECON, FLUX_HLL, true>(P, members, blocks, s) : launch_line_one<R, RECON, FLUX_HLL, false>(P, members, blocks, s);
+    case FLUX_HLL3: return rk3 ? launch_line_one<R, RECON, FLUX_HLL3, true>(P, members, blocks, s) : launch_line_one<R, RECON, FLUX_HLL3, false>(P, members, blocks, s);
+    case FLUX_CENTRAL: return rk3 ? launch_line_one<R, RECON, FLUX_CENTRAL, true>(P, members, blocks, s) : launch_line_one<R, RECON, FLUX_CENTRAL, false>(P, members, blocks, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template<class R>
+cudaError_t launch_line(int recon, int flux, bool rk3, const LineParams& P, int members,
+    int blocks, cudaStream_t s) {
+    switch (recon) {
+    case RECON_NONE: return launch_line_flux<R, RECON_NONE>(flux, rk3, P, members, blocks, s);
+    case RECON_WENO2: return launch_line_flux<R, RECON_WENO2>(flux, rk3, P, members, blocks, s);
+    case RECON_ENO2: return launch_line_flux<R, RECON_ENO2>(flux, rk3, P, members, blocks, s);
+    case RECON_ENO3: return launch_line_flux<R, RECON_ENO3>(flux, rk3, P, members, blocks, s);
+    case RECON_ENO4: return launch_line_flux<R, RECON_ENO4>(flux, rk3, P, members, blocks, s);
+    case RECON_MC: return launch_line_flux<R, RECON_MC>(flux, rk3, P, members, blocks, s);
+    case RECON_MM: return launch_line_flux<R, RECON_MM>(flux, rk3, P, members, blocks, s);
+    case RECON_WENOF2: return launch_line_flux<R, RECON_WENOF2>(flux, rk3, P, members, blocks, s);
+    case RECON_WENO3: return launch_line_flux<R, RECON_WENO3>(flux, rk3, P, members, blocks, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 // Cells per work item of kernel `shape` (0 0 0 when it is not built for the
 // dimension; the runs of the marching rows are split further by the host).
 template<int DIM>
@@ -198,6 +255,8 @@ cudaError_t launch_stage_f64_3d(int recon, int flux, int kind, int shape, const 
 cudaError_t launch_stage_f32_1d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
 cudaError_t launch_stage_f32_2d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
 cudaError_t launch_stage_f32_3d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
+cudaError_t launch_line_f64(int recon, int flux, bool rk3, const LineParams& P, int members, int blocks, cudaStream_t s);
+cudaError_t launch_line_f32(int recon, int flux, bool rk3, const LineParams& P, int members, int blocks, cudaStream_t s);
 void stage_tile_f64_1d(int shape, int* tile);
 void stage_tile_f64_2d(int shape, int* tile);
 void stage_tile_f64_3d(int shape, int* tile);

@@ -10,4 +10,9 @@ cudaError_t launch_stage_f64_1d(int recon, int flux, int kind, int shape,
 void stage_tile_f64_1d(int shape, int* tile) {
     stage_tile_dim<1>(shape, tile);
 }
+cudaError_t launch_line_f64(int recon, int flux, bool rk3, const LineParams& P, int members,
+    int blocks, cudaStream_t s) {
+    return launch_line<double>(recon, flux, rk3, P, members, blocks, s);
+}
+
 } // namespace als

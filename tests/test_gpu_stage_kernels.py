@@ -4,7 +4,8 @@ oracle bit for bit, at the sizes where they can go wrong.
 2-D grids above 400,000 cells (FP64) march warps along y (runs of rows, strips
 of 32 columns), those below 72,000 and 3-D grids below 60,000 take a thread per
 face, 2-D grids between take 16 x 16 tiles, larger 3-D grids march blocks along z
-(segments of planes, 16 x 16 columns).
+(segments of planes, 16 x 16 columns), 1-D RK2 / RK3 runs whole steps in a
+cluster per line.
 """
 import numpy as np
 import pytest
@@ -105,3 +106,59 @@ def test_marching_steps(c_oracle, dim, n, integ, bc):
         info = sim.info()
         np.testing.assert_array_equal(sim.get_state()[0], expect)
     assert info["steps"] == steps and info["t"] == t
+
+
+LINES = [4, 9, 63, 64, 127, 128, 129, 255, 256, 511, 513, 1000, 2047, 4097, 8192, 8193]
+
+
+@pytest.mark.parametrize("n", LINES)
+@pytest.mark.parametrize("integ", ["rungekutta3", "rungekutta2"])
+@pytest.mark.parametrize("bc", ["periodic", "neumann"])
+def test_lines(c_oracle, n, integ, bc):
+    states = np.stack([smooth_random_state(n + m, 1, (n,), 2) for m in range(3)])
+    cfg = c_oracle.config(1, (n,), [0.0], [1.0], "hll3", "weno2", integ, bc, 1.4)
+    end = 0.4 / n
+    runs = [c_oracle.simulate(cfg, s, 0.4, end) for s in states]
+    with als.Simulator(1, (n,), flux="hll3", reconstruction="weno2", integrator=integ, boundary=bc,
+                       cfl=0.4, end_time=end, members=3) as sim:
+        sim.set_state(states)
+        sim.advance(1)          # steps split over calls
+        sim.run()
+        got = sim.get_state()
+        for m, (rc, expect, dts, steps, t) in enumerate(runs):
+            info = sim.info(m)
+            assert info["steps"] == steps and info["t"] == t and info["dt"] == dts[-1]
+            np.testing.assert_array_equal(got[m], expect)
+
+
+@pytest.mark.parametrize("recon", RECONS)
+@pytest.mark.parametrize("flux", ["hll", "hll3"])
+def test_line_schemes(c_oracle, recon, flux):
+    n, g = 300, ghost_cells(recon, flux)
+    st = smooth_random_state(len(recon), 1, (n,), g)
+    cfg = c_oracle.config(1, (n,), [0.0], [1.0], flux, recon, "rungekutta3", "neumann", 1.4)
+    rc, expect, dts, steps, t = c_oracle.simulate(cfg, st, 0.4, 1.0, max_steps=4)
+    with als.Simulator(1, (n,), flux=flux, reconstruction=recon, integrator="rungekutta3",
+                       boundary="neumann", cfl=0.4, end_time=1.0, max_steps=4) as sim:
+        sim.set_state(st)
+        sim.run()
+        assert sim.info()["steps"] == steps
+        np.testing.assert_array_equal(sim.get_state()[0], expect)
+
+
+def test_line_constraint_violation_reports_the_first_cell(c_oracle):
+    n = 700
+    st = smooth_random_state(1, 1, (n,), 2)
+    st[-1, ..., 400:403] = 1e-3           # negative pressure
+    cfg = c_oracle.config(1, (n,), [0.0], [1.0], "hll", "weno2", "rungekutta3", "periodic", 1.4)
+    rc, expect, dts, steps, t = c_oracle.simulate(cfg, st, 0.4, 0.1)
+    with als.Simulator(1, (n,), flux="hll", reconstruction="weno2", cfl=0.4, end_time=0.1,
+                       members=2) as sim:
+        good = smooth_random_state(2, 1, (n,), 2)
+        sim.set_state(np.stack([good, st]))
+        with pytest.raises(als._lib.AlsError):
+            sim.run()
+        bad, fine = sim.info(1), sim.info(0)
+    assert rc != 0 and bad["status"] != 0 and bad["steps"] == steps and bad["bad_step"] == steps
+    assert 380 < bad["bad_index"] < 430
+    assert fine["status"] == 0 and fine["t"] == 0.1
