@@ -303,7 +303,12 @@ __global__ void __launch_bounds__(256) region_sums(const R* states, long long pl
 // running FP64 (n_prev, mean, m2) of every element (Chan et al.'s pairwise
 // update): chunk mean and chunk M2 in FP64, then
 //   n = n_prev + k, d = mean_k - mean, mean += d*k/n, m2 += m2_k + d*d*n_prev*k/n.
-template<class R>
+// K > 0: exactly K members, whose values a thread keeps in registers between
+// the two passes, so that each state is read once and all its loads are in
+// flight together (the two sums add in the same order either way).
+// 256 FP32 states of 4 x 260^2 into a new accumulator: 1.38 -> 0.16 ms (with the
+// pooled accumulator of als_stats_create).
+template<class R, int K>
 __global__ void __launch_bounds__(256) welford_merge(const R* states, long long count,
     int members, long long member_stride, double* mean, double* m2, long long n_prev) {
     const double k = double(members);
@@ -311,14 +316,32 @@ __global__ void __launch_bounds__(256) welford_merge(const R* states, long long 
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
          i += (long long)gridDim.x * blockDim.x) {
         double s = 0;
-        for (int j = 0; j < members; ++j) {
-            s += double(states[(long long)j * member_stride + i]);
-        }
-        const double cm = s / k;
-        double cm2 = 0;
-        for (int j = 0; j < members; ++j) {
-            const double d = double(states[(long long)j * member_stride + i]) - cm;
-            cm2 += d * d;
+        double cm, cm2 = 0;
+        if constexpr (K > 0) {
+            R value[K];
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                value[j] = states[(long long)j * member_stride + i];
+            }
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                s += double(value[j]);
+            }
+            cm = s / k;
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                const double d = double(value[j]) - cm;
+                cm2 += d * d;
+            }
+        } else {
+            for (int j = 0; j < members; ++j) {
+                s += double(states[(long long)j * member_stride + i]);
+            }
+            cm = s / k;
+            for (int j = 0; j < members; ++j) {
+                const double d = double(states[(long long)j * member_stride + i]) - cm;
+                cm2 += d * d;
+            }
         }
         const double d = cm - mean[i];
         mean[i] = mean[i] + d * (k / n);

@@ -364,6 +364,15 @@ cudaError_t scratch_free(void* ptr, cudaStream_t stream) {
     return cudaFreeAsync(ptr, stream);
 }
 
+void scratch_bound() {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long reserved = 0;
+    if (scratch_pool(&pool) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        reserved > kScratchKeep) {
+        cudaMemPoolTrimTo(pool, kScratchKeep);
+    }
+}
 } // namespace als
 
 extern "C" {
@@ -1939,17 +1948,24 @@ struct als_stats {
     int device = 0;
     long long count = 0;          // elements per state
     long long n = 0;              // states accumulated
-    double* mean = nullptr;
+    double* mean = nullptr;       // one allocation for both arrays
     double* m2 = nullptr;
+    bool pooled = false;
     ~als_stats() {
+        if (!mean) {
+            return;
+        }
         int prev = 0;
         cudaGetDevice(&prev);
         cudaSetDevice(device);
-        if (mean) {
+        if (pooled) {
+            // work on any stream may still use the arrays (cudaFree, which the
+            // larger ones take, waits for it too)
+            cudaDeviceSynchronize();
+            als::scratch_free(mean, nullptr);
+            als::scratch_bound();
+        } else {
             cudaFree(mean);
-        }
-        if (m2) {
-            cudaFree(m2);
         }
         cudaSetDevice(prev);
     }
@@ -1960,12 +1976,14 @@ namespace {
 template<class R>
 int stats_merge_states(als_stats* st, const R* states, int members, long long member_stride,
     cudaStream_t s) {
-    // chunks of at most 64 states keep each chunk's two passes in L2
+    // chunks of at most 64 states: a whole one stays in registers between
+    // its two passes, the last one in L2
     for (int first = 0; first < members; first += 64) {
         const int k = std::min(64, members - first);
-        als::welford_merge<R><<<grid_blocks(st->count, 256), 256, 0, s>>>(
-            states + (long long)first * member_stride, st->count, k, member_stride, st->mean, st->m2,
-            st->n);
+        auto merge = k == 64 ? als::welford_merge<R, 64> : als::welford_merge<R, 0>;
+        const long long blocks = std::min<long long>((st->count + 255) / 256, 1LL << 20);
+        merge<<<int(blocks), 256, 0, s>>>(states + (long long)first * member_stride, st->count, k,
+            member_stride, st->mean, st->m2, st->n);
         ALS_CUDA(cudaGetLastError());
         st->n += k;
     }
@@ -1988,10 +2006,19 @@ int als_stats_create(long long count, int device, als_stats** out) {
     st->device = device;
     st->count = count;
     DeviceGuard guard(device);
-    ALS_CUDA(cudaMalloc((void**)&st->mean, sizeof(double) * count));
-    ALS_CUDA(cudaMalloc((void**)&st->m2, sizeof(double) * count));
-    ALS_CUDA(cudaMemset(st->mean, 0, sizeof(double) * count));
-    ALS_CUDA(cudaMemset(st->m2, 0, sizeof(double) * count));
+    // accumulators up to 64 MiB come from the library's pool: a cudaMalloc and
+    // cudaFree per accumulator cost more than adding a few hundred states
+    const size_t bytes = 2 * sizeof(double) * size_t(count);
+    st->pooled = bytes <= (64u << 20);
+    if (st->pooled) {
+        ALS_CUDA(als::scratch_alloc((void**)&st->mean, bytes, nullptr));
+    } else {
+        ALS_CUDA(cudaMalloc((void**)&st->mean, bytes));
+    }
+    st->m2 = st->mean + count;
+    ALS_CUDA(cudaMemsetAsync(st->mean, 0, bytes, nullptr));
+    // the first addition may come on any stream
+    ALS_CUDA(cudaStreamSynchronize(nullptr));
     *out = st.release();
     return ALS_OK;
 }

@@ -162,3 +162,22 @@ def test_line_constraint_violation_reports_the_first_cell(c_oracle):
     assert rc != 0 and bad["status"] != 0 and bad["steps"] == steps and bad["bad_step"] == steps
     assert 380 < bad["bad_index"] < 430
     assert fine["status"] == 0 and fine["t"] == 0.1
+
+
+@pytest.mark.parametrize("precision,bar", [("fp64", 1e-14), ("fp32", 1e-14)])
+@pytest.mark.parametrize("members", [1, 63, 64, 65, 128, 130])
+def test_statistics_chunks(precision, bar, members):
+    """Whole chunks of 64 states stay in registers; mean and variance against
+    two-pass FP64 sums (each a sum of at most 130 terms: 130 x 2^-53)."""
+    dtype = torch.float64 if precision == "fp64" else torch.float32
+    g = torch.Generator().manual_seed(members)
+    states = (3.0 + torch.randn(members, 4, 5, 777, generator=g, dtype=torch.float64)).to(dtype).cuda()
+    mv = als.MeanVariance(states[0].numel())
+    mv.add(states, precision)
+    mean = torch.empty(states.shape[1:], dtype=torch.float64, device="cuda")
+    var = torch.empty_like(mean)
+    mv.result(mean, var)
+    mv.close()
+    x = states.double()
+    assert float((mean - x.mean(0)).abs().max()) < 130 * bar
+    assert float((var - x.var(0, unbiased=False)).abs().max()) < 130 * bar
