@@ -16,14 +16,14 @@
 // So the reconstructed states and fluxes stay in registers, there is no
 // block barrier.  FP64 WENO2 + HLL3, per cell and stage: 690 FP64 instructions
 // of 1,310 (the tiled kernel with plain divisions: 895 of 2,650); FP64 pipe
-// 55 % busy.  Ms per RK3 step: KH 1024^2 FP64 0.279 (tiled) -> 0.244, 512 x
-// 256^2 FP32 members 4.35 -> 2.70; 4096^2 FP64 2.97 (tiled with plain divisions
-// 4.66).
+// 60 % busy; FP32 per cell 730, of the issue slots 80 %.  Ms per RK3 step: KH
+// 1024^2 FP64 0.279 (tiled) -> 0.235, 4096^2 4.66 (tiled, plain divisions) -> 2.83,
+// 512 x 256^2 FP32 members 4.35 -> 2.21.
 //
-// Measured and not taken: x and y interleaved for more independent work per
-// lane (0.258; it spills at 128 registers, and 12 warps per SM with 168 give
-// 0.248), 20 warps per SM at 96 registers (0.272, spills), 12 at 160 (0.242 to
-// 0.251).
+// Measured (KH 1024^2): 12 warps per SM with 166 registers 0.235, 16 with 128
+// 0.235 (spills, and 1 to 2 % slower on larger grids), 18 with 96 0.260; x and y
+// interleaved for more independent work per lane 0.248 to 0.258; forming U1
+// as the rows are loaded instead of as they are stored 0.248.
 //
 // The arithmetic and its order are those of stage_kernel, so the results are
 // its bits.
@@ -51,7 +51,7 @@ struct RowLayout {
 };
 
 #ifndef ALS_ROWS_WARPS64
-#define ALS_ROWS_WARPS64 16
+#define ALS_ROWS_WARPS64 12
 #endif
 #ifndef ALS_ROWS_WARPS32
 #define ALS_ROWS_WARPS32 24
@@ -136,9 +136,6 @@ __device__ __forceinline__ void rows_tile(const StageParams& P, const LevelDesc&
     }
 
     const int g = gd.ghosts;
-    auto input = [&](int v, long long cell) {
-        return StageInputFetch<R, KIND>{&L, cell, c}.at(v, 0);
-    };
 
     R wmax[2] = {R(0), R(0)};
     bool bad = false;
@@ -182,32 +179,52 @@ __device__ __forceinline__ void rows_tile(const StageParams& P, const LevelDesc&
         const int col = x0 + lane;
         const bool in_region = col < gd.hi[0];
         R* mine = ring + S + lane;       // this lane's column in slot 0
-        // the ring's columns of this lane: x0 + lane - S and, in its tail, 32
-        // further; lanes and rows beyond the grid read its last column or
-        // row, ordinary values whose results nobody uses
+        // One row of the stage's input, as loaded (U1 is formed when the row goes
+        // into the ring, a row later, so that nothing waits for its loads): this
+        // lane's column x0 + lane - S, and one value of the 2 S columns after the
+        // warp's, one lane per variable and column.  Columns and rows beyond the
+        // grid read its last one: ordinary values whose results nobody uses.
+        struct Row {
+            R in[NV], un[NV], tin, tun;
+        };
+        const bool tail = S > 0 && lane < 2 * S * NV;
+        const int tv = tail ? lane / (S > 0 ? 2 * S : 1) : 0;
+        const int tk = 32 + (tail ? lane % (S > 0 ? 2 * S : 1) : 0);
         const int pa = min(x0 + lane - S + g, gd.N[0] - 1);
-        const int pb = min(x0 + lane - S + 32 + g, gd.N[0] - 1);
-        auto fetch_row = [&](int y, R* a, R* b) {
+        const int pt = min(x0 + tk - S + g, gd.N[0] - 1);
+        const R* tail_in = static_cast<const R*>(L.in[tv]);
+        const R* tail_un = static_cast<const R*>(L.un[tv]);
+        auto fetch_row = [&](int y, Row& r) {
             const long long first = base + (long long)min(y + g, gd.N[1] - 1) * gd.N[0];
-            const long long ia = first + pa;
-            const long long ib = first + pb;
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                a[v] = input(v, ia);
-                b[v] = R(0);
-                if (S > 0 && lane < 2 * S) {
-                    b[v] = input(v, ib);
+                r.in[v] = static_cast<const R*>(L.in[v])[first + pa];
+                if (FORMS) {
+                    r.un[v] = static_cast<const R*>(L.un[v])[first + pa];
+                }
+            }
+            if (tail) {
+                r.tin = tail_in[first + pt];
+                if (FORMS) {
+                    r.tun = tail_un[first + pt];
                 }
             }
         };
-        auto store_row = [&](int slot, const R* a, const R* b) {
-            R* dst = ring + slot * Lay::ROW + lane;
+        auto formed = [&](R in, R un) {
+            if (FORMS) {
+                in = in * c;
+                in = in + un;
+            }
+            return in;
+        };
+        auto store_row = [&](int slot, const Row& r) {
+            R* dst = ring + slot * Lay::ROW;
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                dst[v * Lay::BX] = a[v];
-                if (S > 0 && lane < 2 * S) {
-                    dst[v * Lay::BX + 32] = b[v];
-                }
+                dst[v * Lay::BX + lane] = formed(r.in[v], r.un[v]);
+            }
+            if (tail) {
+                dst[tv * Lay::BX + tk] = formed(r.tin, r.tun);
             }
         };
         auto next = [](int s) { return s + 1 == Lay::RING ? 0 : s + 1; };
@@ -215,25 +232,26 @@ __device__ __forceinline__ void rows_tile(const StageParams& P, const LevelDesc&
 
         // rows j0-1-S .. j0-1+S into slots 0 .. 2S: the cell below the run,
         // then the first cell and the face between them
-        R a[NV], b[NV], ry[NV], fy[NV];
+        R ry[NV], fy[NV];
+        Row ahead;
 #pragma unroll
         for (int k = 0; k < 2 * S + 1; ++k) {
-            fetch_row(j0 - 1 - S + k, a, b);
-            store_row(k, a, b);
+            fetch_row(j0 - 1 - S + k, ahead);
+            store_row(k, ahead);
         }
         int centre = S;                  // slot of the row reconstructed along y
         int fill = (2 * S + 1) % Lay::RING;   // slot the next row goes to
-        fetch_row(j0 + S, a, b);
+        fetch_row(j0 + S, ahead);
         __syncwarp();
         {
             R l[NV];
             reconstruct_f<R, NV, RECON>(Column{mine, centre}, l, ry, gamma);
         }
         __syncwarp();
-        store_row(fill, a, b);
+        store_row(fill, ahead);
         fill = next(fill);
         centre = next(centre);
-        fetch_row(j0 + 1 + S, a, b);
+        fetch_row(j0 + 1 + S, ahead);
         __syncwarp();
         {
             R l[NV], r[NV];
@@ -252,13 +270,13 @@ __device__ __forceinline__ void rows_tile(const StageParams& P, const LevelDesc&
         for (int j = j0; j < j1; ++j) {
             // row j + 1 + S replaces the oldest; the one after it is on its way
             __syncwarp();
-            store_row(fill, a, b);
+            store_row(fill, ahead);
             fill = next(fill);
             const int here = centre;     // slot of row j
             centre = next(centre);
             __syncwarp();
             if (j + 1 < j1) {
-                fetch_row(j + 2 + S, a, b);
+                fetch_row(j + 2 + S, ahead);
             }
             R un[NV];
             if (in_region) {
