@@ -138,15 +138,27 @@ int grid_for(long long work, int threads) {
     return int(b < 1 ? 1 : (b > 148LL * 16 ? 148LL * 16 : b));
 }
 
+// `chained`: the stream's last kernel produces this one's operands and the
+// launch may overlap its end (the kernel waits for it before it reads).
 template <int BN, int EPI>
-int launch_gemm(const GemmArgs& a, int n_valid, cudaStream_t s, int splits = 1) {
+int launch_gemm(const GemmArgs& a, int n_valid, cudaStream_t s, int splits = 1,
+                bool chained = false) {
     if (a.M % kTileM || a.N % BN || a.K % kChunkK || a.K <= 0 || splits < 1 || splits > 65535) {
         return mlp_fail(ALS_E_INVALID, "GEMM shape is not a multiple of the tile");
     }
     constexpr int smem = gemm_smem_bytes<BN>();   // limit set by configure_kernels()
     dim3 grid(a.M / kTileM, a.N / BN, splits);
-    gemm_kernel<BN, EPI><<<grid, kThreads, smem, s>>>(a, n_valid);
-    MLP_CUDA(cudaGetLastError());
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = dim3(kThreads);
+    config.dynamicSmemBytes = smem;
+    config.stream = s;
+    config.attrs = &overlap;
+    config.numAttrs = chained ? 1 : 0;
+    MLP_CUDA(cudaLaunchKernelEx(&config, gemm_kernel<BN, EPI>, a, n_valid));
     return ALS_OK;
 }
 
@@ -315,7 +327,7 @@ int forward_hidden(als_mlp* s, const __nv_bfloat16* x, long long rows_pad,
                              : (launch_tma_forward<4, false>(ta, s->tm_w[l], a, hw, hb, nullptr, 0, st)));
             }
         } else if (zs || L.out % 128 != 0) {
-            MLP_TRY((launch_gemm<64, EPI_FORWARD>(a, L.out, st)));
+            MLP_TRY((launch_gemm<64, EPI_FORWARD>(a, L.out, st, 1, zs && l > 0)));
         } else if (L.out % 256 != 0) {
             MLP_TRY((launch_gemm<128, EPI_FORWARD>(a, L.out, st)));
         } else {
@@ -390,7 +402,8 @@ int k_splits(long long K) {
 // do; the weight and bias gradients of a layer hang on its dZ alone and run
 // on the two side streams meanwhile (each layer with buffers of its own), and
 // their partial products are added where they are used.  One training step at
-// batch 1024, 40 -> 256 x 4 -> 1: 0.237 -> 0.150 ms.
+// batch 1024, 40 -> 256 x 4 -> 1 (of a long call): 0.208 ms one after another,
+// 0.087 so, 0.068 with the GEMMs' staging and epilogue in whole rows.
 int enqueue_gradients(als_mlp* s, const float* t, int rows, float* loss, long long base,
                       Gradient* grad, cudaEvent_t begun, cudaStream_t st) {
     const int nh = s->cfg.hidden;
@@ -427,7 +440,7 @@ int enqueue_gradients(als_mlp* s, const float* t, int rows, float* loss, long lo
             b.ldz = L.in;
             b.ldh = L.in;
             arm(s, b);
-            MLP_TRY((launch_gemm<64, EPI_BACKWARD>(b, L.in, st)));
+            MLP_TRY((launch_gemm<64, EPI_BACKWARD>(b, L.in, st, 1, true)));
         }
         for (int k = 0; k < 2; ++k) {
             MLP_CUDA(cudaStreamWaitEvent(s->branch[k], s->dz_ready[l], 0));
@@ -861,23 +874,41 @@ int als_mlp_train(als_mlp* s, const float* x_dev, const float* t_dev, int rows, 
 
     // the inputs do not change between the steps of a call
     MLP_TRY(pack_batch(s, x_dev, rows, st));
+    // blocks of Adam for the largest range, a weight matrix
+    const long long most = (long long)s->cfg.width * std::max(s->cfg.width, s->cfg.inputs);
+    const unsigned adam_blocks = unsigned((most + 255) / 256);
+    auto enqueue_step = [&]() -> int {
+        MLP_CUDA(cudaEventRecord(s->branch_done[0], st));
+        MLP_CUDA(cudaStreamWaitEvent(s->branch[1], s->branch_done[0], 0));
+        begin_step<<<1, 1, 0, s->branch[1]>>>(s->step, loss_dev, base);
+        MLP_CUDA(cudaGetLastError());
+        MLP_CUDA(cudaEventRecord(s->branch_done[1], s->branch[1]));
+        MLP_TRY(enqueue_gradients(s, t_dev, rows, loss_dev, base, &a.g, s->branch_done[1], st));
+        adam_update<<<dim3(adam_blocks, unsigned(a.g.ranges)), 256, 0, st>>>(a);
+        MLP_CUDA(cudaGetLastError());
+        return ALS_OK;
+    };
+    // capturing and instantiating the step's graph takes as long as about ten
+    // steps, and launching the kernels one by one nearly keeps up with them:
+    // the graph pays from some fifty steps on
+    if (steps < 64) {
+        int rc = ALS_OK;
+        for (int k = 0; k < steps && rc == ALS_OK; ++k) {
+            rc = enqueue_step();
+        }
+        const cudaError_t se = cudaStreamSynchronize(st);
+        if (rc != ALS_OK) {
+            return rc;
+        }
+        if (se != cudaSuccess) {
+            return mlp_fail(ALS_E_CUDA, std::string("training step: ") + cudaGetErrorString(se));
+        }
+        return check_error_flag(s);
+    }
     // one training step, captured once and replayed
     cudaGraph_t graph = nullptr;
     MLP_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    int rc = ALS_OK;
-    if (cudaEventRecord(s->branch_done[0], st) != cudaSuccess ||
-        cudaStreamWaitEvent(s->branch[1], s->branch_done[0], 0) != cudaSuccess) {
-        rc = mlp_fail(ALS_E_CUDA, "training step: fork failed");
-    }
-    begin_step<<<1, 1, 0, s->branch[1]>>>(s->step, loss_dev, base);
-    if (rc == ALS_OK && cudaEventRecord(s->branch_done[1], s->branch[1]) != cudaSuccess) {
-        rc = mlp_fail(ALS_E_CUDA, "training step: fork failed");
-    }
-    rc = rc != ALS_OK ? rc : enqueue_gradients(s, t_dev, rows, loss_dev, base, &a.g,
-                                               s->branch_done[1], st);
-    if (rc == ALS_OK) {
-        adam_update<<<grid_for(s->nparams, 256), 256, 0, st>>>(a);
-    }
+    const int rc = enqueue_step();
     const cudaError_t ce = cudaStreamEndCapture(st, &graph);
     if (rc != ALS_OK || ce != cudaSuccess) {
         if (graph) {

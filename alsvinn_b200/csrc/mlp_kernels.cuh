@@ -21,58 +21,61 @@ constexpr int gemm_smem_bytes() {
     return gemm_stages<BN>() * (kTileM * kChunkK * 2 + BN * kChunkK * 2) + 1024;
 }
 
-template <int BN, int EPI>
-__device__ __forceinline__ void epilogue16(const GemmArgs& g, long long m, int n, const float* v,
-                                           int n_valid) {
+// The epilogue of a wide inference tile (BN > 64): 16 columns of one row.
+__device__ __forceinline__ void epilogue16(const GemmArgs& g, long long m, int n, const float* v) {
+    __align__(16) __nv_bfloat16 hb[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        hb[i] = __float2bfloat16_rn(gelu_half(fmaf(0.5f, v[i], 0.5f * g.bias[n + i])));
+    }
+    uint4* dh = reinterpret_cast<uint4*>(g.h + m * g.ldh + n);
+    dh[0] = reinterpret_cast<const uint4*>(hb)[0];
+    dh[1] = reinterpret_cast<const uint4*>(hb)[1];
+}
+
+// The epilogue of a 128 x 64 training tile through shared memory: a thread
+// holds one row of the accumulator, so writing from there would send every
+// store of a warp to 32 rows; a warp instead takes whole rows, a lane columns
+// `lane` and `lane + 32`.  `tile` has rows of 65 floats.
+constexpr int kTileLd = 65;
+
+// `zin`: the pre-activations of this thread's rows and columns, loaded while
+// the MMAs run (EPI_BACKWARD).
+constexpr int kTileRows = kTileM / (kThreads / 32);     // rows per warp
+
+template <int EPI>
+__device__ __forceinline__ void epilogue_rows(const GemmArgs& g, const float* tile, const float* zin,
+                                              long long m0, int n0, int n_valid) {
+    const int lane = threadIdx.x & 31;
+    const int na = n0 + lane, nb = na + 32;
+    float ba = 0.0f, bb = 0.0f;
     if (EPI == EPI_FORWARD) {
-        if (g.z) {
-            __align__(16) float z[16];
+        ba = g.bias[na];
+        bb = g.bias[nb];
+    }
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                z[i] = v[i] + g.bias[n + i];
+    for (int i = 0; i < kTileRows; ++i) {
+        const int r = (threadIdx.x >> 5) + i * (kThreads / 32);
+        const float va = tile[r * kTileLd + lane];
+        const float vb = tile[r * kTileLd + lane + 32];
+        const long long m = m0 + r;
+        if (EPI == EPI_FORWARD) {
+            if (g.z) {
+                g.z[m * g.ldz + na] = va + ba;
+                g.z[m * g.ldz + nb] = vb + bb;
             }
-            float4* dz = reinterpret_cast<float4*>(g.z + m * g.ldz + n);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                dz[i] = reinterpret_cast<const float4*>(z)[i];
-            }
-        }
-        __align__(16) __nv_bfloat16 hb[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            hb[i] = __float2bfloat16_rn(gelu_half(fmaf(0.5f, v[i], 0.5f * g.bias[n + i])));
-        }
-        uint4* dh = reinterpret_cast<uint4*>(g.h + m * g.ldh + n);
-        dh[0] = reinterpret_cast<const uint4*>(hb)[0];
-        dh[1] = reinterpret_cast<const uint4*>(hb)[1];
-    } else if (EPI == EPI_BACKWARD) {
-        __align__(16) float zin[16];
-        const float4* sz = reinterpret_cast<const float4*>(g.zin + m * g.ldz + n);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            reinterpret_cast<float4*>(zin)[i] = sz[i];
-        }
-        __align__(16) __nv_bfloat16 hb[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            hb[i] = __float2bfloat16_rn(v[i] * gelu_grad(zin[i]));
-        }
-        uint4* dh = reinterpret_cast<uint4*>(g.h + m * g.ldh + n);
-        dh[0] = reinterpret_cast<const uint4*>(hb)[0];
-        dh[1] = reinterpret_cast<const uint4*>(hb)[1];
-    } else {
-        float* dst = g.g + blockIdx.z * g.split_stride + m * g.ldg + n;
-        if (n + 16 <= n_valid && (g.ldg & 3) == 0) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                reinterpret_cast<float4*>(dst)[i] = make_float4(v[4 * i], v[4 * i + 1],
-                                                                v[4 * i + 2], v[4 * i + 3]);
-            }
+            g.h[m * g.ldh + na] = __float2bfloat16_rn(gelu_half(fmaf(0.5f, va, 0.5f * ba)));
+            g.h[m * g.ldh + nb] = __float2bfloat16_rn(gelu_half(fmaf(0.5f, vb, 0.5f * bb)));
+        } else if (EPI == EPI_BACKWARD) {
+            g.h[m * g.ldh + na] = __float2bfloat16_rn(va * gelu_grad(zin[2 * i]));
+            g.h[m * g.ldh + nb] = __float2bfloat16_rn(vb * gelu_grad(zin[2 * i + 1]));
         } else {
-            for (int i = 0; i < 16; ++i) {
-                if (n + i < n_valid) {
-                    dst[i] = v[i];
-                }
+            float* dst = g.g + blockIdx.z * g.split_stride + m * g.ldg;
+            if (na < n_valid) {
+                dst[na] = va;
+            }
+            if (nb < n_valid) {
+                dst[nb] = vb;
             }
         }
     }
@@ -84,7 +87,8 @@ __device__ __forceinline__ void epilogue16(const GemmArgs& g, long long m, int n
 // `n_valid` limits the stored columns of EPI_WGRAD (padded inputs).
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid) {
-    static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "TMEM columns: power of two");
+    static_assert(BN == 64 || ((BN == 128 || BN == 256) && EPI == EPI_FORWARD),
+                  "training tiles are 64 wide; wider ones infer (no Z kept)");
     constexpr int kStages = gemm_stages<BN>();
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t bars[kStages];
@@ -104,6 +108,9 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
     const long long n0 = (long long)blockIdx.y * BN;
     const int kb = blockIdx.z * g.K;
 
+    // the next GEMM of a training step may take its place and set itself up
+    // while this one runs
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == 0) {
         tmem_alloc(&tmem_base, BN);
     }
@@ -120,6 +127,8 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
     const uint32_t tmem = tmem_base;
     const uint32_t idesc = instr_desc_bf16(kTileM, BN);
     const int nk = g.K / kChunkK;
+    // operands come from the kernel before (a no-op unless launched so)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // the MMAs of chunk c from stage st
     auto issue = [&](int c, int st) {
@@ -134,10 +143,8 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
     int last = -1;          // last chunk whose MMAs were committed
     bool failed = false;
     if (nk <= kStages) {
-        for (int c = 0; c < nk; ++c) {
-            stage_operand<kTileM>(sa(c), g.a, m0, kb + c * kChunkK);
-            stage_operand<BN>(sb(c), g.b, n0, kb + c * kChunkK);
-        }
+        stage_operand<kTileM>(sa(0), kABytes + kBBytes, g.a, m0, kb, nk);
+        stage_operand<BN>(sb(0), kABytes + kBBytes, g.b, n0, kb, nk);
         stage_wait();
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -161,8 +168,8 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
                 failed = true;
                 break;
             }
-            stage_operand<kTileM>(sa(s), g.a, m0, kb + c * kChunkK);
-            stage_operand<BN>(sb(s), g.b, n0, kb + c * kChunkK);
+            stage_operand<kTileM>(sa(s), 0, g.a, m0, kb + c * kChunkK, 1);
+            stage_operand<BN>(sb(s), 0, g.b, n0, kb + c * kChunkK, 1);
             stage_wait();
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -173,6 +180,15 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
                 }
             }
             last = c;
+        }
+    }
+    float zin[2 * kTileRows];
+    if (BN == 64 && EPI == EPI_BACKWARD) {
+#pragma unroll
+        for (int i = 0; i < kTileRows; ++i) {
+            const float* z = g.zin + (m0 + warp + i * (kThreads / 32)) * g.ldz + n0 + lane;
+            zin[2 * i] = z[0];
+            zin[2 * i + 1] = z[32];
         }
     }
     bool done = false;
@@ -191,13 +207,29 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid)
         // warp w reads TMEM lane quarter w % 4, half w / 4 of the columns
         const int quarter = warp & 3;
         const int first = (warp >> 2) * (BN / 2);
-        const long long m = m0 + quarter * 32 + lane;
+        const int row = quarter * 32 + lane;
         const uint32_t lane_base = tmem + (uint32_t(quarter * 32) << 16);
+        if (BN == 64) {
+            // the operands are consumed: their memory takes the tile
+            float* tile = reinterpret_cast<float*>(base);
+#pragma unroll
+            for (int c0 = 0; c0 < BN / 2; c0 += 16) {
+                float v[16];
+                tmem_load16(lane_base + uint32_t(first + c0), v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    tile[row * kTileLd + first + c0 + i] = v[i];
+                }
+            }
+            __syncthreads();
+            epilogue_rows<EPI>(g, tile, zin, m0, int(n0), n_valid);
+        } else {
 #pragma unroll 1
-        for (int c0 = first; c0 < first + BN / 2; c0 += 16) {
-            float v[16];
-            tmem_load16(lane_base + uint32_t(c0), v);
-            epilogue16<BN, EPI>(g, m, int(n0) + c0, v, n_valid);
+            for (int c0 = first; c0 < first + BN / 2; c0 += 16) {
+                float v[16];
+                tmem_load16(lane_base + uint32_t(c0), v);
+                epilogue16(g, m0 + row, int(n0) + c0, v);
+            }
         }
     }
     tc_fence_before();
@@ -393,7 +425,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_forward(const __grid_
                                                make_float2(head_w[c0 + i], head_w[c0 + i + 1]), hsum2);
                         }
                     } else {
-                        epilogue16<BN, EPI_FORWARD>(g, m, c0, v, BN);
+                        epilogue16(g, m, c0, v);
                     }
                 }
                 tc_fence_before();
@@ -958,27 +990,37 @@ struct AdamArgs {
     int nseg;
 };
 
-__global__ void adam_update(AdamArgs a) {
-    const long long t = a.step[0];
-    const float c1 = 1.0f - powf(a.beta1, float(t));
-    const float c2 = 1.0f - powf(a.beta2, float(t));
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const float gi = a.g.at(i);
+// Grid: x over the elements, y over the ranges of the parameter vector.
+__global__ void __launch_bounds__(256) adam_update(AdamArgs a) {
+    __shared__ float corr[2];
+    if (threadIdx.x < 2) {
+        corr[threadIdx.x] = 1.0f - powf(threadIdx.x ? a.beta2 : a.beta1, float(a.step[0]));
+    }
+    __syncthreads();
+    const float c1 = corr[0];
+    const float c2 = corr[1];
+    const GradRange& r = a.g.range[blockIdx.y];
+    // the range of a hidden weight matrix keeps a BF16 copy up to date
+    const int layer = blockIdx.y >> 1;
+    const bool copied = (blockIdx.y & 1) == 0 && layer < a.nseg;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < r.count; j += gridDim.x * blockDim.x) {
+        const float* part = r.partial + j;
+        float gi = 0.0f;
+#pragma unroll 8
+        for (int k = 0; k < r.splits; ++k) {
+            gi += part[k * r.count];
+        }
+        const long long i = r.first + j;
         const float mi = a.beta1 * a.m[i] + (1.0f - a.beta1) * gi;
         const float vi = a.beta2 * a.v[i] + (1.0f - a.beta2) * gi * gi;
         a.m[i] = mi;
         a.v[i] = vi;
         const float pi = a.p[i] - a.lr * (mi / c1) / (sqrtf(vi / c2) + a.eps);
         a.p[i] = pi;
-        for (int s = 0; s < a.nseg; ++s) {
-            const Segment& sg = a.seg[s];
-            const long long rel = i - sg.w_off;
-            if (sg.wb && rel >= 0 && rel < (long long)sg.out * sg.in) {
-                const long long o = rel / sg.in;
-                const int k = int(rel - o * sg.in);
-                sg.wb[o * sg.kpad + k] = __float2bfloat16_rn(pi);
-            }
+        if (copied) {
+            const Segment& sg = a.seg[layer];
+            const int o = j / sg.in;
+            sg.wb[o * sg.kpad + (j - o * sg.in)] = __float2bfloat16_rn(pi);
         }
     }
 }

@@ -263,34 +263,60 @@ __device__ __forceinline__ void stage_wait() {
     fence_async_shared();
 }
 
-// Stages rows [row0, row0+ROWS) x K [k0, k0+64) of an operand into `dst`;
-// 16-byte aligned rows when K is contiguous.
+// Stages rows [row0, row0+ROWS) x K [k0, k0 + 64 chunks) of an operand, chunk
+// c into `base` + c * stride; 16-byte aligned rows when K is contiguous.  The
+// work of all chunks is dealt to the threads at once, so that their loads are
+// in flight together.
 template <int ROWS>
-__device__ __forceinline__ void stage_operand(unsigned char* dst, const Operand& op, long long row0,
-                                              int k0) {
+__device__ __forceinline__ void stage_operand(unsigned char* base, int stride, const Operand& op,
+                                              long long row0, int k0, int chunks) {
     if (op.ks == 1) {
-        // rows of contiguous K: one 16-byte vector per (row, 8-wide K group)
-        for (int idx = threadIdx.x; idx < ROWS * 8; idx += kThreads) {
-            const int r = idx >> 3;
-            const int kc = idx & 7;
+        // rows of contiguous K: one 16-byte vector per (row, 8-wide K group);
+        // a warp takes 8 rows x 4 groups, so that each quarter of it fills 128
+        // contiguous bytes of shared memory
+        for (int idx = threadIdx.x; idx < ROWS * 8 * chunks; idx += kThreads) {
+            const int c = idx / (ROWS * 8);
+            const int r = ((idx >> 6) & (ROWS / 8 - 1)) * 8 + (idx & 7);
+            const int kc = (idx >> 3) & 7;
             // asynchronous: complete after stage_wait
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
-                         ::"r"(smem_u32(dst + staged_offset(r, kc))),
-                           "l"(op.p + (row0 + r) * op.rs + k0 + kc * 8)
+                         ::"r"(smem_u32(base + c * stride + staged_offset(r, kc))),
+                           "l"(op.p + (row0 + r) * op.rs + k0 + c * kChunkK + kc * 8)
                          : "memory");
         }
     } else {
-        // transposed operand: consecutive rows are contiguous in memory
-        for (int idx = threadIdx.x; idx < ROWS * 8; idx += kThreads) {
-            const int r = idx % ROWS;
-            const int kc = idx / ROWS;
-            const __nv_bfloat16* src = op.p + (row0 + r) * op.rs + (long long)(k0 + kc * 8) * op.ks;
-            __align__(16) __nv_bfloat16 e[8];
+        // transposed operand, its rows contiguous (rs = 1, ks a multiple of 8): 8 x 8
+        // blocks, 8 loads of 8 rows each, exchanged in registers
+        for (int idx = threadIdx.x; idx < ROWS * chunks; idx += kThreads) {
+            unsigned char* dst = base + idx / ROWS * stride;
+            const int r0 = (idx % (ROWS / 8)) * 8;
+            const int kc = (idx / (ROWS / 8)) & 7;
+            const __nv_bfloat16* src = op.p + row0 + r0 +
+                (long long)(k0 + idx / ROWS * kChunkK + kc * 8) * op.ks;
+            uint4 in[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                e[j] = src[(long long)j * op.ks];
+                in[j] = *reinterpret_cast<const uint4*>(src + (long long)j * op.ks);
             }
-            *reinterpret_cast<uint4*>(dst + staged_offset(r, kc)) = *reinterpret_cast<uint4*>(e);
+            // word w of in[j]: rows 2w, 2w + 1 at k = j; each lane starts at
+            // another pair, as equal rows of all blocks share their banks
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+                const int w = (it + idx) & 3;
+                uint32_t x[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint32_t lo = (w & 1) ? in[j].y : in[j].x;
+                    const uint32_t hi = (w & 1) ? in[j].w : in[j].z;
+                    x[j] = (w & 2) ? hi : lo;
+                }
+                const uint4 even = make_uint4(__byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410),
+                                              __byte_perm(x[4], x[5], 0x5410), __byte_perm(x[6], x[7], 0x5410));
+                const uint4 odd = make_uint4(__byte_perm(x[0], x[1], 0x7632), __byte_perm(x[2], x[3], 0x7632),
+                                             __byte_perm(x[4], x[5], 0x7632), __byte_perm(x[6], x[7], 0x7632));
+                *reinterpret_cast<uint4*>(dst + staged_offset(r0 + 2 * w, kc)) = even;
+                *reinterpret_cast<uint4*>(dst + staged_offset(r0 + 2 * w + 1, kc)) = odd;
+            }
         }
     }
 }
