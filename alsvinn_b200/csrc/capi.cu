@@ -136,7 +136,8 @@ int run_rows(long long strip_rows, int precision) {
 
 // Planes per segment of the 3-D blocks that march along z, for a launch of
 // `column_planes` planes of 16 x 16 cells in all: as run_rows, with about one
-// plane lost per segment and two resident blocks per SM.  FP64, ms: KH 128^3 x 2,
+// plane lost per segment and two resident blocks per SM.  FP64, ms (16 x 16 columns): KH
+// 128^3 x 2,
 // 4 steps, segments of 32 planes 8.29, 12 7.64, 8 7.50, 5 7.80, 2 9.11; 64^3, 16
 // steps, 16 planes 7.45, 8 4.35, 4 2.62, 2 2.92.
 int segment_planes(long long column_planes) {
@@ -194,7 +195,7 @@ int choose_kernel(int dim, int flux, int shape, long long cells, int precision) 
         cells <= kTilesCells2[precision == ALS_FP64 ? 0 : 1]) {
         return 1;
     }
-    return shape;
+    return dim == 3 && shape == 1 ? als::kPlanesKernel : shape;
 }
 
 // The tile shape a configuration starts on: in 3-D the columns marching along

@@ -70,7 +70,7 @@ inline cudaError_t launch_stage_blocks(void (*kernel)(StageParams), int threads,
 
 // The kernel of one (kernel id, kind): a thread per face for id kFacesKernel
 // and for 1-D two-point fluxes; in 2-D id 0 with a two-point flux the warps
-// marching along y; in 3-D id 1 the columns marching along z; else the tiled
+// marching along y; id kPlanesKernel the columns marching along z; else the tiled
 // stage_kernel of that shape.
 template<class R, int DIM, int RECON, int FLUX, int KIND, int SHAPE>
 cudaError_t launch_stage_one(const StageParams& P, int b, cudaStream_t s) {
@@ -78,7 +78,7 @@ cudaError_t launch_stage_one(const StageParams& P, int b, cudaStream_t s) {
         typedef FaceLayout<R, DIM, RECON, FLUX> Lay;
         return launch_stage_blocks(faces_kernel<R, DIM, RECON, FLUX, KIND>, Lay::THREADS, Lay::SMEM,
             P, b, s);
-    } else if constexpr (DIM == 3 && SHAPE == 1) {
+    } else if constexpr (SHAPE == kPlanesKernel) {
         typedef ZLayout<R, RECON, FLUX> Lay;
         return launch_stage_blocks(zmarch_kernel<R, RECON, FLUX, KIND>, Lay::THREADS, Lay::SMEM, P,
             b, s);
@@ -111,6 +111,11 @@ cudaError_t launch_stage_shape(int kernel, int kind, const StageParams& P, int b
     if constexpr (kernel_built(DIM, RECON, FLUX, kFacesKernel)) {
         if (kernel == kFacesKernel) {
             return launch_stage_kind<R, DIM, RECON, FLUX, kFacesKernel>(kind, P, b, s);
+        }
+    }
+    if constexpr (kernel_built(DIM, RECON, FLUX, kPlanesKernel)) {
+        if (kernel == kPlanesKernel) {
+            return launch_stage_kind<R, DIM, RECON, FLUX, kPlanesKernel>(kind, P, b, s);
         }
     }
     if constexpr (kernel_built(DIM, RECON, FLUX, 0)) {
@@ -229,6 +234,11 @@ void stage_tile_dim(int shape, int* tile) {
         tile[0] = FaceBox<DIM>::X;
         tile[1] = FaceBox<DIM>::Y;
         tile[2] = FaceBox<DIM>::Z;
+    }
+    if (shape == kPlanesKernel && DIM == 3) {
+        tile[0] = kColumnsX;
+        tile[1] = kColumnsY;
+        tile[2] = ALS_ZMARCH_SEG;
     }
     if (shape == 0) {
         tile[0] = TileShape<DIM, 0>::X;

@@ -123,23 +123,17 @@ template<> struct TileShape<3, 0> {
     static constexpr int X = ALS_TILE3_X, Y = ALS_TILE3_Y, Z = ALS_TILE3_Z, T = ALS_STAGE3_THREADS,
         B = ALS_STAGE3_BLOCKS;
 };
-// 3-D shape 1: 16 x 16 columns marching along z over segments of
-// ALS_ZMARCH_SEG cells (stage_zmarch.cuh), 288 threads (96 registers at two
-// blocks per SM).  KH 128^3 x 8, FP64, ms per RK3 step: 10.59 (segments of
-// 16: 10.66; 320 threads: 10.60; 256 threads, 128 registers but two rounds
-// per x-y phase: 12.17), against 12.40 for the 8x8x4 boxes.
+// 3-D shape 1: columns marching along z (stage_zmarch.cuh).  This is its
+// nominal tile; the kernel's own columns and segments are chosen there and by
+// the host.
 #ifndef ALS_ZMARCH_SEG
 #define ALS_ZMARCH_SEG 32
 #endif
 #ifndef ALS_ZMARCH_BLOCKS
 #define ALS_ZMARCH_BLOCKS 2
 #endif
-#ifndef ALS_ZMARCH_THREADS
-#define ALS_ZMARCH_THREADS 288
-#endif
 template<> struct TileShape<3, 1> {
-    static constexpr int X = 16, Y = 16, Z = ALS_ZMARCH_SEG, T = ALS_ZMARCH_THREADS,
-        B = ALS_ZMARCH_BLOCKS;
+    static constexpr int X = 16, Y = 16, Z = ALS_ZMARCH_SEG;
 };
 
 // Shapes built per (dimension, reconstruction, flux): the default for every
@@ -158,7 +152,9 @@ constexpr int kMaxShapes = 2;
 // The kernel that runs a level's stages: that of its tile shape, or
 // kFacesKernel, one thread per face (stage_faces.cuh).
 constexpr int kFacesKernel = 2;
-constexpr int kMaxKernels = 3;
+// 3-D shape 1 is run by blocks of other columns than its nominal tile
+constexpr int kPlanesKernel = 3;
+constexpr int kMaxKernels = 4;
 
 // Two-point fluxes have it in every dimension; in 1-D it is the only one.  In
 // 2-D the 16 x 16 tiles also serve levels of shape 0 (als_solver_set_tiles
@@ -166,6 +162,8 @@ constexpr int kMaxKernels = 3;
 // reconstruction.
 __host__ __device__ constexpr bool kernel_built(int dim, int recon, int flux, int kernel) {
     return kernel == kFacesKernel ? !stencil_flux(flux)
+        : kernel == kPlanesKernel ? dim == 3 && shape_built(dim, recon, flux, 1)
+        : dim == 3 && kernel == 1 ? false
         : (dim == 2 && kernel == 1 && flux <= FLUX_CENTRAL) ||
             (shape_built(dim, recon, flux, kernel) && (dim > 1 || stencil_flux(flux)));
 }
@@ -177,7 +175,7 @@ __host__ __device__ constexpr bool marches_rows(int dim, int flux, int kernel) {
 
 // Whether they are segments of planes (stage_zmarch.cuh).
 __host__ __device__ constexpr bool marches_planes(int dim, int kernel) {
-    return dim == 3 && kernel == 1;
+    return dim == 3 && kernel == kPlanesKernel;
 }
 
 template<class R, int DIM, int RECON, int FLUX, int SHAPE = 0>

@@ -19,6 +19,9 @@ constexpr int kMaxLevels = 4;
 // the warps marching along y (stage_rows.cuh): columns, and most rows, of a run
 constexpr int kRunColumns = 32;
 constexpr int kRunRows = 32;
+// the blocks marching along z (stage_zmarch.cuh): columns of a block
+constexpr int kColumnsX = 16;
+constexpr int kColumnsY = 15;
 
 // Per-simulation time-stepping state kept on the device, so a whole time
 // step runs without a host round trip.  One per ensemble member.

@@ -1,15 +1,21 @@
 // 3-D stage kernel that marches along z (tile shape 1 of the 3-D stage).
 //
-// A block owns a 16 x 16 column of cells over a segment of at most
-// ALS_ZMARCH_SEG cells along z (the host chooses the length).  It keeps a ring of three x-y planes (each with its x-y halo of
-// G cells, every conserved variable) in shared memory and walks the segment
-// plane by plane.  Per plane, the x and y directions reconstruct and
-// evaluate their faces like the 2-D kernel; then the thread of each column
+// A block owns a 16 x 15 column of cells over a segment of at most
+// ALS_ZMARCH_SEG cells along z (the host chooses the length).  It keeps a ring
+// of three x-y planes (each with its x-y halo of G cells, every conserved
+// variable) in shared memory and walks the segment plane by plane.  Per plane
+// every x face and then every y face has a thread, which reconstructs both of
+// its sides and evaluates the flux; then the thread of each column
 // reconstructs the next cell of its column along z and evaluates the z face
 // between the two, keeping that face's flux and the next cell's right state
-// (in shared memory, private to the column) for the next plane.  So every cell is reconstructed along z once and every
-// z face is evaluated once, where the 8 x 8 x 4 tiles of shape 0 reconstruct
-// 1.5 cells per cell along z and stage a box of 4.5 times the tile.
+// (in shared memory, private to the column) for the next plane.  So every cell
+// is reconstructed along z once and every z face is evaluated once, where the
+// 8 x 8 x 4 tiles of shape 0 reconstruct 1.5 cells per cell along z and stage a
+// box of 4.5 times the tile.  The columns are 16 x 15 so that 255 x faces, 256 y
+// faces and 240 columns fill 256 threads, which leaves FP64 128 registers at
+// two blocks per SM.  KH 128^3 x 2, FP64, 4 RK3 steps: 6.72 ms, with 16 x 16
+// columns, 288 threads and each cell reconstructed once per direction through
+// shared memory (six barriers a plane instead of three) 7.65.
 //
 // The arithmetic and its order are those of stage_kernel (the same
 // reconstruction, flux and update_cell; the net flux of a cell adds its x,
@@ -24,28 +30,27 @@ namespace als {
 
 template<class R, int RECON, int FLUX>
 struct ZLayout {
-    typedef TileShape<3, 1> Shape;
     static constexpr int NV = 5;
     static constexpr int G = stage_ghosts(RECON, FLUX);
     static constexpr int S = recon_ghosts(RECON) - 1;   // stencil half-width along z
-    static constexpr int TX = Shape::X;
-    static constexpr int TY = Shape::Y;
+    static constexpr int TX = kColumnsX;
+    static constexpr int TY = kColumnsY;
     static constexpr int BX = TX + 2 * G;
     static constexpr int BY = TY + 2 * G;
     static constexpr int PLANE = BX * BY;
     static constexpr int RING = 3;
     static constexpr int COLS = TX * TY;
-    static constexpr int THREADS = Shape::T;
-    static constexpr int REC = (TX + 2) * TY > TX * (TY + 2) ? (TX + 2) * TY : TX * (TY + 2);
-    static constexpr int FAC = (TX + 1) * TY > TX * (TY + 1) ? (TX + 1) * TY : TX * (TY + 1);
-    // ring, x-y reconstructions, x-y face fluxes, and per column the right
-    // state below the next z face and the flux through the face below
+    static constexpr int THREADS = 256;
+    static constexpr int FACX = (TX + 1) * TY;
+    static constexpr int FACY = TX * (TY + 1);
+    // ring, x and y face fluxes, and per column the right state below the next
+    // z face and the flux through the face below
     static constexpr size_t SMEM = sizeof(R) *
-        (size_t(NV) * PLANE * RING + size_t(2 * NV) * REC + size_t(NV) * FAC + size_t(2 * NV) * COLS);
-    static constexpr int BY_SMEM = int((228 * 1024) / (SMEM + 1024));
-    static constexpr int BLOCKS = BY_SMEM < 1 ? 1 : (BY_SMEM > Shape::B ? Shape::B : BY_SMEM);
+        (size_t(NV) * PLANE * RING + size_t(NV) * (FACX + FACY) + size_t(2 * NV) * COLS);
+    static constexpr int BLOCKS = ALS_ZMARCH_BLOCKS;
     static_assert(S == 0 || S == 1, "the ring holds a stencil of one cell each way along z");
-    static_assert(COLS <= THREADS && THREADS % 32 == 0, "one thread per column, whole warps");
+    static_assert(COLS <= THREADS && FACX <= THREADS && FACY <= THREADS, "a thread per column and face");
+    static_assert(BLOCKS * (SMEM + 1024) <= 228 * 1024, "the blocks share the SM's memory");
 };
 
 // Values of one column at planes kc-1, kc, kc+1 of the ring (the fetcher of
@@ -62,87 +67,45 @@ struct ColumnFetch {
     __device__ __forceinline__ R dyn(int v, int o) const { return at(v, o); }
 };
 
-// The x (D = 0) or y (D = 1) direction of plane `pl`: reconstruct every cell
-// its faces need, evaluate every face once, and add each column's net flux
-// into that column's thread's acc (as stage_direction does for a tile).
+// The x (D = 0) or y (D = 1) faces of plane `pl`, a thread each: both sides
+// reconstructed (they share their smoothness terms) and the flux into
+// flx[v * faces + i].
 template<class R, int RECON, int FLUX, int KIND, int D>
-__device__ __forceinline__ void plane_direction(const GridDesc& gd, R gamma, const R* pl, R* rec,
-    R* flx, R* acc, R& wmax, int x0, int y0) {
+__device__ __forceinline__ void plane_faces(const GridDesc& gd, R gamma, const R* pl, R* flx,
+    R& wmax, int x0, int y0) {
     typedef ZLayout<R, RECON, FLUX> Lay;
     constexpr int NV = Lay::NV;
-    constexpr int G = Lay::G;
-    constexpr int E0 = Lay::TX + (D == 0 ? 2 : 0);
-    constexpr int E1 = Lay::TY + (D == 1 ? 2 : 0);
-    constexpr int RC = E0 * E1;
     constexpr int F0 = Lay::TX + (D == 0 ? 1 : 0);
-    constexpr int F1 = Lay::TY + (D == 1 ? 1 : 0);
-    constexpr int FC = F0 * F1;
+    constexpr int FC = D == 0 ? Lay::FACX : Lay::FACY;
     constexpr int ST = D == 0 ? 1 : Lay::BX;
-    const int tid = threadIdx.x;
-
-    for (int i = tid; i < RC; i += Lay::THREADS) {
-        const int ex = i % E0;
-        const int ey = i / E0;
-        const int bx = ex - (D == 0 ? 1 : 0) + G;
-        const int by = ey - (D == 1 ? 1 : 0) + G;
-        R l[NV], r[NV];
-        reconstruct<R, NV, RECON>(pl + by * Lay::BX + bx, Lay::PLANE, ST, l, r, gamma);
+    const int i = threadIdx.x;
+    if (i >= FC) {
+        return;
+    }
+    const int fx = i % F0;
+    const int fy = i / F0;
+    const R* right = pl + (fy + Lay::G) * Lay::BX + fx + Lay::G;
+    const StridedFetch<R, int> fl{right - ST, Lay::PLANE, ST};
+    const StridedFetch<R, int> fr{right, Lay::PLANE, ST};
+    R ul[NV], ur[NV], skip[NV], F[NV];
+    bool okl, okr;
+    reconstruct_d<R, NV, RECON, true>(fl, skip, ul, gamma, okl);
+    reconstruct_d<R, NV, RECON, true>(fr, ur, skip, gamma, okr);
+    if (!okl || !okr) {
+        reconstruct_f<R, NV, RECON>(fl, skip, ul, gamma);
+        reconstruct_f<R, NV, RECON>(fr, ur, skip, gamma);
+    }
+    const R w = face_flux_best<R, 3, FLUX, D>(ul, ur, gamma, F);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            rec[v * RC + i] = l[v];
-            rec[(NV + v) * RC + i] = r[v];
+    for (int v = 0; v < NV; ++v) {
+        flx[v * FC + i] = F[v];
+    }
+    if (KIND == KIND_FLUX0) {
+        const bool valid = x0 + fx - (D == 0 ? 1 : 0) < gd.hi[0] && y0 + fy - (D == 1 ? 1 : 0) < gd.hi[1];
+        if (valid && wmax < w) {
+            wmax = w;
         }
     }
-    __syncthreads();
-
-    const int hiD = D == 0 ? gd.hi[0] : gd.hi[1];
-    const int oD = D == 0 ? x0 : y0;
-    for (int i = tid; i < FC; i += Lay::THREADS) {
-        const int fx = i % F0;
-        const int fy = i / F0;
-        const int rl = fy * E0 + fx;
-        const int rr = rl + (D == 0 ? 1 : E0);
-        R ul[NV], ur[NV], F[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            ul[v] = rec[(NV + v) * RC + rl];
-            ur[v] = rec[v * RC + rr];
-        }
-        const R w = face_flux_best<R, 3, FLUX, D>(ul, ur, gamma, F);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            flx[v * FC + i] = F[v];
-        }
-        if (KIND == KIND_FLUX0) {
-            const int f = D == 0 ? fx : fy;
-            bool valid = oD + f - 1 <= hiD - 1;
-            if (D != 0) {
-                valid = valid && (x0 + fx < gd.hi[0]);
-            }
-            if (D != 1) {
-                valid = valid && (y0 + fy < gd.hi[1]);
-            }
-            if (valid && wmax < w) {
-                wmax = w;
-            }
-        }
-    }
-    __syncthreads();
-
-    if (tid < Lay::COLS) {
-        const int cx = tid % Lay::TX;
-        const int cy = tid / Lay::TX;
-        const int fl = cy * F0 + cx;
-        const int fr = fl + (D == 0 ? 1 : F0);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const R tr = -flx[v * FC + fr];
-            const R tl = -flx[v * FC + fl];
-            acc[v] = acc[v] + (tr + (-tl));
-        }
-    }
-    // no barrier: the next writer of flx is the next face phase, behind the
-    // barrier that ends the next reconstruction
 }
 
 // One work item: columns (tx, ty) over z segment tz of member `member`.
@@ -158,10 +121,10 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
     StepState* st = L.state ? L.state + (L.subdomains ? 0 : member) : nullptr;
 
     R* ring = reinterpret_cast<R*>(smem);
-    R* rec = ring + Lay::RING * NV * Lay::PLANE;
-    R* flx = rec + 2 * NV * Lay::REC;
+    R* flx = ring + Lay::RING * NV * Lay::PLANE;
+    R* fly = flx + NV * Lay::FACX;
     // column-private: Rk[v] = zs[v * COLS + col], Fm[v] = zs[(NV + v) * COLS + col]
-    R* zs = flx + NV * Lay::FAC;
+    R* zs = fly + NV * Lay::FACY;
 
     const int tx = tile % gd.tiles[0];
     const int ty = (tile / gd.tiles[0]) % gd.tiles[1];
@@ -277,15 +240,23 @@ __device__ __forceinline__ void zmarch_tile(const StageParams& P, const LevelDes
         __syncthreads();
         load_plane(k + 2);
         __syncthreads();
-        R acc[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            acc[v] = R(0);
-        }
         const R* pl = slot(k);
-        plane_direction<R, RECON, FLUX, KIND, 0>(gd, gamma, pl, rec, flx, acc, wmax[0], x0, y0);
-        plane_direction<R, RECON, FLUX, KIND, 1>(gd, gamma, pl, rec, flx, acc, wmax[1], x0, y0);
+        plane_faces<R, RECON, FLUX, KIND, 0>(gd, gamma, pl, flx, wmax[0], x0, y0);
+        plane_faces<R, RECON, FLUX, KIND, 1>(gd, gamma, pl, fly, wmax[1], x0, y0);
+        __syncthreads();
         if (column) {
+            R acc[NV];
+            const int xl = cy * (Lay::TX + 1) + cx;
+            const int yl = cy * Lay::TX + cx;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const R xr = -flx[v * Lay::FACX + xl + 1];
+                const R xf = -flx[v * Lay::FACX + xl];
+                acc[v] = R(0) + (xr + (-xf));
+                const R yr = -fly[v * Lay::FACY + yl + Lay::TX];
+                const R yf = -fly[v * Lay::FACY + yl];
+                acc[v] = acc[v] + (yr + (-yf));
+            }
             // z: the face above the cell, between it and the next cell up
             R l[NV], r[NV], rb[NV], Fp[NV];
             recon_z(k + 1, l, r);

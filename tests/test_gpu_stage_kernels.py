@@ -4,7 +4,7 @@ oracle bit for bit, at the sizes where they can go wrong.
 2-D grids above 400,000 cells (FP64) march warps along y (runs of rows, strips
 of 32 columns), those below 72,000 and 3-D grids below 60,000 take a thread per
 face, 2-D grids between take 16 x 16 tiles, larger 3-D grids march blocks along z
-(segments of planes, 16 x 16 columns), 1-D RK2 / RK3 runs whole steps in a
+(segments of planes, 16 x 15 columns), 1-D RK2 / RK3 runs whole steps in a
 cluster per line.
 """
 import numpy as np
