@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <sstream>
 #include <string>
+#include <type_traits>
 
 #include "als_b200.h"
 #include "scratch.h"
@@ -230,8 +231,10 @@ __global__ void __launch_bounds__(kThreads) structure_kernel(const T* __restrict
 // difference, so the two FP64 operations of a difference are what binds.
 // On a torus |u(x) - u(x + d)| summed over all x is the same for d and -d:
 // with periodic boundaries one of each pair is walked and counted twice.
-// 32 x 256^2 FP32 states, H = 8, p = 1, periodic: 1.46 -> 0.36 ms (0.94e9
-// differences, 2.6e12 a second; the FP64 pipe's bound is 9.3e12).
+// 32 x 256^2 FP32 states, H = 8, p = 1, periodic: 1.46 -> 0.31 ms (0.94e9
+// differences, 3.0e12 a second; the FP64 pipe's bound is 9.3e12); 0.36 with
+// cells beyond the grid masked in every strip instead of the last, 0.34 at 72
+// registers (fewer warps) instead of 64.
 template<int DIM> struct CubeTile;
 // The largest tile; the host halves y, then z, until the blocks fill the GPU.
 template<> struct CubeTile<2> { static constexpr int X = 32, Y = 64, Z = 1; };
@@ -244,7 +247,9 @@ __global__ void __launch_bounds__(kThreads) structure_cube_kernel(const T* __res
     long long member_stride, StructGeom G, int nvar, int H, double p, double* __restrict__ partial) {
     constexpr bool HALF = BC == ALS_BC_PERIODIC;
     constexpr int COLS = 4;              // cells per thread and strip
-    constexpr int W = COLS + 2 * (HM - 1);
+    // least y offset walked: a torus in 2-D needs none below the row
+    constexpr int LO = HALF && DIM == 2 ? 0 : 1 - HM;
+    constexpr int W = COLS + HM - 1 - LO;
     extern __shared__ double box[];
     __shared__ double part[kWarps][HM];
     const int member = blockIdx.z;
@@ -292,44 +297,52 @@ __global__ void __launch_bounds__(kThreads) structure_cube_kernel(const T* __res
         for (int k = 0; k < COLS; ++k) {
             uc[k] = centre[k * bx];
         }
-        for (int dz = DIM > 2 ? (HALF ? 0 : -R) : 0; dz <= (DIM > 2 ? R : 0); ++dz) {
-            for (int dx = (SHARE ? team : 0) - R; dx <= R; dx += SHARE ? teams : 1) {
-                // y offsets from `first`: with HALF and dz = 0 only half the plane
-                const int first = HALF && dz == 0 ? (dx > 0 ? 0 : 1) : -R;
-                const int far = max(abs(dx), abs(dz));
-                const double* col = centre + dz * (by * bx) + dx;
-                double w[W];
+        // every strip but the grid's last holds four cells
+        auto walk = [&](auto whole) {
+            for (int dz = DIM > 2 ? (HALF ? 0 : -R) : 0; dz <= (DIM > 2 ? R : 0); ++dz) {
+                for (int dx = (SHARE ? team : 0) - R; dx <= R; dx += SHARE ? teams : 1) {
+                    // y offsets from `first`: with HALF and dz = 0 only half the plane
+                    const int first = HALF && dz == 0 ? (dx > 0 ? 0 : 1) : -R;
+                    const int far = max(abs(dx), abs(dz));
+                    const double* col = centre + dz * (by * bx) + dx;
+                    double w[W];
 #pragma unroll
-                for (int k = 0; k < W; ++k) {
-                    const int dy = k - (HM - 1);   // row offset from the first cell
-                    w[k] = dy >= first && dy <= R + COLS - 1 ? col[dy * bx] : 0.0;
-                }
-                double near = 0;                  // the offsets whose cube is `far`
-#pragma unroll
-                for (int dy = -(HM - 1); dy <= HM - 1; ++dy) {
-                    if (dy < first || dy > R) {
-                        continue;
+                    for (int k = 0; k < W; ++k) {
+                        const int dy = k + LO;   // row offset from the first cell
+                        w[k] = dy >= first && dy <= R + COLS - 1 ? col[dy * bx] : 0.0;
                     }
-                    double d = 0;
+                    double near = 0;                  // the offsets whose cube is `far`
 #pragma unroll
-                    for (int k = 0; k < COLS; ++k) {
-                        const double t = spow<P>(fabs(uc[k] - w[k + dy + HM - 1]), p);
-                        d += k < left ? t : 0.0;
-                    }
-                    const int a = dy < 0 ? -dy : dy;
-                    if (a > far) {
-                        acc[a] += d;
-                    } else {
-                        near += d;
-                    }
-                }
+                    for (int dy = LO; dy < HM; ++dy) {
+                        if (dy < first || dy > R) {
+                            continue;
+                        }
+                        double d = 0;
 #pragma unroll
-                for (int h = 1; h < HM; ++h) {
-                    if (h == far) {
-                        acc[h] += near;
+                        for (int k = 0; k < COLS; ++k) {
+                            const double t = spow<P>(fabs(uc[k] - w[k + dy - LO]), p);
+                            d += decltype(whole)::value || k < left ? t : 0.0;
+                        }
+                        const int a = dy < 0 ? -dy : dy;
+                        if (a > far) {
+                            acc[a] += d;
+                        } else {
+                            near += d;
+                        }
+                    }
+#pragma unroll
+                    for (int h = 1; h < HM; ++h) {
+                        if (h == far) {
+                            acc[h] += near;
+                        }
                     }
                 }
             }
+        };
+        if (left == COLS) {
+            walk(std::true_type());
+        } else {
+            walk(std::false_type());
         }
     }
 #pragma unroll
