@@ -138,6 +138,16 @@ int grid_for(long long work, int threads) {
     return int(b < 1 ? 1 : (b > 148LL * 16 ? 148LL * 16 : b));
 }
 
+// The inputs of `rows` rows (a chunk or a batch) rounded and padded into xb.
+void launch_pack(const float* x, long long rows, int nin, __nv_bfloat16* xb, long long rows_pad,
+                 int kpad, cudaStream_t st) {
+    const int units = (nin + 7) / 8;
+    const dim3 block(units, 256 / units);
+    const int wide = nin % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+    pack_inputs<<<unsigned((rows_pad + block.y - 1) / block.y), block, 0, st>>>(
+        x, int(rows), nin, wide, xb, int(rows_pad), kpad);
+}
+
 // `chained`: the stream's last kernel produces this one's operands and the
 // launch may overlap its end (the kernel waits for it before it reads).
 template <int BN, int EPI>
@@ -485,8 +495,7 @@ int enqueue_gradients(als_mlp* s, const float* t, int rows, float* loss, long lo
 int pack_batch(als_mlp* s, const float* x, int rows, cudaStream_t st) {
     const long long rp = round_up(rows, kTileM);
     const Layer& L0 = s->layers[0];
-    pack_inputs<<<grid_for(rp * (L0.kpad / 8), 256), 256, 0, st>>>(x, rows, s->cfg.inputs, s->xb, rp,
-                                                             L0.kpad);
+    launch_pack(x, rows, s->cfg.inputs, s->xb, rp, L0.kpad, st);
     MLP_CUDA(cudaGetLastError());
     if (rp > rows) {
         const size_t W = size_t(s->cfg.width);
@@ -556,8 +565,8 @@ int forward_fused_chunks(als_mlp* s, const float* x_dev, long long rows, float* 
         if (i >= 2) {
             MLP_CUDA(cudaStreamWaitEvent(s->side, s->xi_free[b], 0));
         }
-        pack_inputs<<<grid_for(rp * (L0.kpad / 8), 256), 256, 0, s->side>>>(
-            x_dev + r0 * s->cfg.inputs, n, s->cfg.inputs, b ? s->xi2 : s->xi, rp, L0.kpad);
+        launch_pack(x_dev + r0 * s->cfg.inputs, n, s->cfg.inputs, b ? s->xi2 : s->xi, rp, L0.kpad,
+                    s->side);
         MLP_CUDA(cudaGetLastError());
         MLP_CUDA(cudaEventRecord(s->packed[b], s->side));
         MLP_CUDA(cudaStreamWaitEvent(st, s->packed[b], 0));
@@ -593,8 +602,7 @@ int forward_rows(als_mlp* s, const float* x_dev, long long rows, float* y_dev, v
     for (long long r0 = 0; r0 < rows; r0 += kInferChunk) {
         const long long n = rows - r0 < kInferChunk ? rows - r0 : kInferChunk;
         const long long rp = (n + kTileM - 1) / kTileM * kTileM;
-        pack_inputs<<<grid_for(rp * (L0.kpad / 8), 256), 256, 0, st>>>(
-            x_dev + r0 * s->cfg.inputs, n, s->cfg.inputs, s->xi, rp, L0.kpad);
+        launch_pack(x_dev + r0 * s->cfg.inputs, n, s->cfg.inputs, s->xi, rp, L0.kpad, st);
         MLP_CUDA(cudaGetLastError());
         const __nv_bfloat16* last = nullptr;
         MLP_TRY(forward_hidden(s, s->xi, rp, nullptr, nullptr, s->hi, &last, st,

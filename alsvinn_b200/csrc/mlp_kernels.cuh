@@ -83,7 +83,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmArgs& g, const float* ti
 
 // D[128 x BN tile] = A * B^T over K, then the epilogue.  Grid: (M/128, N/BN,
 // splits): split z covers K range [z K, (z+1) K) and, with EPI_WGRAD, writes
-// its partial product z * split_stride further (summed by sum_splits).
+// its partial product z * split_stride further (Gradient::at adds them).
 // `n_valid` limits the stored columns of EPI_WGRAD (padded inputs).
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g, int n_valid) {
@@ -801,23 +801,46 @@ __global__ void __launch_bounds__(kTmaThreads) mlp_forward_fused(const __grid_co
     }
 }
 
-// x (rows x nin, FP32) -> xb (rows_pad x kpad, BF16), zero padded; one
-// 16-byte store of 8 values per work item.
-__global__ void pack_inputs(const float* __restrict__ x, long long rows, int nin,
-                            __nv_bfloat16* __restrict__ xb, long long rows_pad, int kpad) {
-    const int groups = kpad >> 3;
-    const long long total = rows_pad * groups;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / groups;
-        const int k0 = int(i - r * groups) * 8;
-        __align__(16) __nv_bfloat16 v[8];
+// x (rows x nin, FP32) -> xb (rows_pad x kpad, BF16): 8 values per thread,
+// written as one 16-byte unit, zeros beyond `nin` and `rows`.  The units of a
+// row that hold inputs only (blockDim.x of them): the others stay the zeros
+// the buffer was allocated with.  With `wide` (rows of whole, aligned 16-byte
+// units) a thread reads its values in two loads.  Bound by memory alone, but
+// it runs beside the network kernel, whose epilogue lacks issue slots: with a
+// 64-bit division and eight single loads per unit, zero units included, 2^20
+// rows of 40 inputs took 0.596 ms per forward call instead of 0.585, 237,762
+// rows of a 128-wide network 0.251 instead of 0.238.
+__global__ void pack_inputs(const float* __restrict__ x, int rows, int nin, int wide,
+                            __nv_bfloat16* __restrict__ xb, int rows_pad, int kpad) {
+    const int k0 = int(threadIdx.x) * 8;
+    const int r = blockIdx.x * blockDim.y + threadIdx.y;
+    if (r < rows_pad) {
+        float v[8] = {};
+        if (r < rows) {
+            const float* row = x + (long long)r * nin;
+            if (wide) {
+                if (k0 < nin) {
+                    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(row + k0);
+                }
+                if (k0 + 4 < nin) {
+                    *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(row + k0 + 4);
+                }
+            } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int k = k0 + j;
-            v[j] = __float2bfloat16_rn((r < rows && k < nin) ? x[r * nin + k] : 0.0f);
+                for (int j = 0; j < 8; ++j) {
+                    if (k0 + j < nin) {
+                        v[j] = row[k0 + j];
+                    }
+                }
+            }
         }
-        *reinterpret_cast<uint4*>(xb + r * kpad + k0) = *reinterpret_cast<const uint4*>(v);
+        __nv_bfloat162 h[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+        }
+        *reinterpret_cast<uint4*>(xb + (long long)r * kpad + k0) =
+            *reinterpret_cast<const uint4*>(h);
     }
 }
 
@@ -898,7 +921,7 @@ __global__ void head_step(const __nv_bfloat16* __restrict__ h, const float* __re
 }
 
 // out[split][n] = sum over rows [split*rows_per_split, ...) of wt[r] * X[r][n]
-// (wt null: weights 1), deterministic order; sum_splits adds the splits.
+// (wt null: weights 1), deterministic order; Gradient::at adds the splits.
 // Block: 32 columns x 8 row groups; grid (columns / 32, splits).
 template <typename T>
 __global__ void column_sums(const T* __restrict__ x, int rows, int cols, long long ld,

@@ -51,6 +51,27 @@ def test_forward_matches_oracle(inputs, width, hidden, rows):
     assert np.abs(y - ref).mean() <= 1e-3 * scale
 
 
+@pytest.mark.parametrize("inputs", [1, 3, 4, 8, 12, 20, 40, 60, 64])
+@pytest.mark.parametrize("rows", [1, 127, 300])
+def test_input_packing_by_wide_and_single_loads(inputs, rows):
+    """Rows of whole 16-byte units are read four values at a time, from an
+    aligned pointer only: the same rows one float further on take single
+    loads and give the same bits, and both match the oracle."""
+    rng = np.random.default_rng(100 * inputs + rows)
+    x = rng.uniform(-1, 1, (rows, inputs)).astype(np.float32)
+    flat = torch.zeros(rows * inputs + 1, dtype=torch.float32, device="cuda")
+    flat[1:] = torch.from_numpy(x.ravel())
+    shifted = flat[1:].view(rows, inputs)
+    with als.Surrogate(inputs, 256, 2, max_batch=512, seed=3) as s:
+        a = s.forward_raw(torch.from_numpy(x).cuda()).cpu().numpy()
+        b = s.forward_raw(shifted).cpu().numpy()
+        p = s.params()
+    assert np.array_equal(a, b)
+    ref, _ = mo.forward(p, x, inputs, 256, 2, bf16_path=True)
+    # as test_forward_matches_oracle: 1e-2 of the output scale
+    assert np.abs(a - ref).max() <= 1e-2 * (np.abs(ref).max() + 1e-3)
+
+
 @pytest.mark.parametrize("rows", [256, 200])
 def test_gradients_match_oracle(rows):
     inputs, width, hidden = 40, 256, 4
