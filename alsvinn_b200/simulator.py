@@ -208,9 +208,9 @@ class Simulator:
     def set_tiles(self, shapes):
         """Tile shape per level: 0 the dimension's box tile (2-D 32x16, 3-D
         8x8x4 cells); 1 the alternative where it is built (2-D 16x16 cells
-        for WENO2 with HLL, HLL3 or Central; 3-D 16x16 columns marching along
-        z, the 3-D default, for reconstructions reaching one cell with the
-        two-point fluxes)."""
+        for WENO2 with HLL, HLL3 or Central; 3-D columns marching along z, the
+        3-D default, for reconstructions reaching one cell with the two-point
+        fluxes).  Nominal: a level's size chooses among the kernels as well."""
         arr = (ctypes.c_int * len(self.levels))(*[int(v) for v in shapes])
         _lib.check(self._lib.als_solver_set_tiles(self._h, arr))
 

@@ -266,8 +266,10 @@ int als_solver_set_schedule(als_solver* s, int blocks_per_sm, const int* level_o
 int als_solver_get_schedule(const als_solver* s, int* blocks_per_sm, int* level_order);
 /* Tile shape of each level's stage kernels: 0 is every dimension's default
  * (1-D 256, 2-D 32x16, 3-D 8x8x4 cells); 2-D WENO2 with HLL, HLL3 or
- * Central also has shape 1 (16x16 cells, 288 threads).  Levels of
- * different shapes take one launch per shape and stage.  The shape changes
+ * Central also has shape 1 (16x16 cells), 3-D its default, columns marching
+ * along z.  The extents are nominal: the kernel that runs a level follows
+ * its size as well.  Levels run by different kernels take one launch per
+ * kernel and stage.  The shape changes
  * no result.  set returns ALS_E_UNSUPPORTED for a shape not built for the
  * configuration; get fills tile_shapes[level] and tile_extents[3*level + d]
  * (either may be NULL). */

@@ -74,8 +74,9 @@ int als_mlp_gradients(als_mlp* h, const float* x_dev, const float* t_dev, int ro
                       float* grad_dev, float* loss, void* stream);
 
 /* `steps` full-batch Adam steps (beta1 0.9, beta2 0.999, eps 1e-8, learning
- * rate `lr`) on the mean squared error over `rows` samples, one CUDA graph
- * per step.  loss_dev (steps floats, or null) receives each step's loss. */
+ * rate `lr`) on the mean squared error over `rows` samples.  Calls
+ * of 64 steps and more replay one captured graph, shorter ones launch the
+ * step's kernels directly.  loss_dev (steps floats, or null) receives each step's loss. */
 int als_mlp_train(als_mlp* h, const float* x_dev, const float* t_dev, int rows, int steps,
                   float lr, float* loss_dev, void* stream);
 
