@@ -633,9 +633,11 @@ __device__ __forceinline__ void write_cell(const StageParams& P, const LevelDesc
         }
     }
     if (check && st && !obeys_constraints<R, NV>(val, gamma)) {
-        bad = true;
         // subdomains: the member's padded plane offset first
-        bad_idx = L.subdomains ? (long long)member * gd.plane + idx : idx;
+        const long long at = L.subdomains ? (long long)member * gd.plane + idx : idx;
+        // the first of this thread's cells, whatever the order it takes them in
+        bad_idx = bad && bad_idx < at ? bad_idx : at;
+        bad = true;
     }
 }
 

@@ -164,6 +164,37 @@ def test_line_constraint_violation_reports_the_first_cell(c_oracle):
     assert fine["status"] == 0 and fine["t"] == 0.1
 
 
+BAD = [(1, (300,), "weno2", "hll3", 1), (2, (40, 30), "weno2", "hll3", 3), (2, (300, 270), "weno2", "hll3", 1),
+       (2, (703, 631), "weno2", "hll3", 1), (2, (200, 100), "none", "tecno4", 2),
+       (3, (20, 18, 16), "weno2", "hll3", 1), (3, (50, 47, 44), "weno2", "hll3", 1),
+       (3, (50, 47, 44), "eno3", "hll3", 1)]
+
+
+@pytest.mark.parametrize("dim,n,recon,flux,members", BAD,
+                         ids=["%s-%s-%s" % ("x".join(map(str, c[1])), c[2], c[3]) for c in BAD])
+def test_reported_cell_is_the_first_violation(dim, n, recon, flux, members):
+    """Several cells of one thread violate the constraints (some columns, over
+    all rows and planes): bad_index is the smallest padded index of them all,
+    in every stage kernel."""
+    g = ghost_cells(recon, flux)
+    states = np.stack([smooth_random_state(17 + m, dim, n, g) for m in range(members)])
+    states[:, -1, :, :, g + n[0] // 3:g + n[0] // 3 + max(3, n[0] // 3)] = 1e-3   # negative pressure
+    with als.Simulator(dim, n, flux=flux, reconstruction=recon, cfl=0.4, end_time=1.0, max_steps=1,
+                       members=members) as sim:
+        sim.set_state(states)
+        with pytest.raises(als._lib.AlsError):
+            sim.run()
+        for m in range(members):
+            U = sim.get_state(m, 1)[0]
+            with np.errstate(all="ignore"):
+                p = (1.4 - 1) * (U[-1] - 0.5 * sum(U[1 + d] * U[1 + d] for d in range(dim)) / U[0])
+                ok = np.isfinite(U).all(0) & (U[0] > 0) & (p > 0)
+            inner = np.zeros(ok.shape, bool)
+            inner[tuple(slice(g, g + n[d]) if d < dim else slice(None) for d in (2, 1, 0))] = True
+            bad = np.flatnonzero(inner & ~ok)
+            assert len(bad) > 1 and sim.info(m)["bad_index"] == bad[0]
+
+
 @pytest.mark.parametrize("precision,bar", [("fp64", 1e-14), ("fp32", 1e-14)])
 @pytest.mark.parametrize("members", [1, 63, 64, 65, 128, 130])
 def test_statistics_chunks(precision, bar, members):
