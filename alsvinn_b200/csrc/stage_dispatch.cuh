@@ -152,21 +152,48 @@ cudaError_t launch_stage_flux(int flux, int kind, int shape, const StageParams& 
     return cudaErrorInvalidValue;
 }
 
-template<class R, int DIM>
-cudaError_t launch_stage_dim(int recon, int flux, int kind, int shape, const StageParams& P, int b,
+// The reconstructions of a translation unit: the 2-D and 3-D kernels of one
+// precision are built in three units, side by side (one alone takes minutes).
+constexpr int kReconGroups = 3;
+constexpr int recon_group(int recon) {
+    return recon == RECON_NONE || recon == RECON_WENO2 || recon == RECON_ENO2 ? 0
+        : (recon == RECON_ENO3 || recon == RECON_ENO4 || recon == RECON_WENO3 ? 1 : 2);
+}
+
+template<class R, int DIM, int GROUP>
+cudaError_t launch_stage_group(int recon, int flux, int kind, int shape, const StageParams& P, int b,
     cudaStream_t s) {
-    switch (recon) {
-    case RECON_NONE: return launch_stage_flux<R, DIM, RECON_NONE>(flux, kind, shape, P, b, s);
-    case RECON_WENO2: return launch_stage_flux<R, DIM, RECON_WENO2>(flux, kind, shape, P, b, s);
-    case RECON_ENO2: return launch_stage_flux<R, DIM, RECON_ENO2>(flux, kind, shape, P, b, s);
-    case RECON_ENO3: return launch_stage_flux<R, DIM, RECON_ENO3>(flux, kind, shape, P, b, s);
-    case RECON_ENO4: return launch_stage_flux<R, DIM, RECON_ENO4>(flux, kind, shape, P, b, s);
-    case RECON_MC: return launch_stage_flux<R, DIM, RECON_MC>(flux, kind, shape, P, b, s);
-    case RECON_MM: return launch_stage_flux<R, DIM, RECON_MM>(flux, kind, shape, P, b, s);
-    case RECON_WENOF2: return launch_stage_flux<R, DIM, RECON_WENOF2>(flux, kind, shape, P, b, s);
-    case RECON_WENO3: return launch_stage_flux<R, DIM, RECON_WENO3>(flux, kind, shape, P, b, s);
-    default: return cudaErrorInvalidValue;
+    if constexpr (GROUP == 0) {
+        switch (recon) {
+        case RECON_NONE: return launch_stage_flux<R, DIM, RECON_NONE>(flux, kind, shape, P, b, s);
+        case RECON_WENO2: return launch_stage_flux<R, DIM, RECON_WENO2>(flux, kind, shape, P, b, s);
+        case RECON_ENO2: return launch_stage_flux<R, DIM, RECON_ENO2>(flux, kind, shape, P, b, s);
+        default: return cudaErrorInvalidValue;
+        }
+    } else if constexpr (GROUP == 1) {
+        switch (recon) {
+        case RECON_ENO3: return launch_stage_flux<R, DIM, RECON_ENO3>(flux, kind, shape, P, b, s);
+        case RECON_ENO4: return launch_stage_flux<R, DIM, RECON_ENO4>(flux, kind, shape, P, b, s);
+        case RECON_WENO3: return launch_stage_flux<R, DIM, RECON_WENO3>(flux, kind, shape, P, b, s);
+        default: return cudaErrorInvalidValue;
+        }
+    } else {
+        switch (recon) {
+        case RECON_MC: return launch_stage_flux<R, DIM, RECON_MC>(flux, kind, shape, P, b, s);
+        case RECON_MM: return launch_stage_flux<R, DIM, RECON_MM>(flux, kind, shape, P, b, s);
+        case RECON_WENOF2: return launch_stage_flux<R, DIM, RECON_WENOF2>(flux, kind, shape, P, b, s);
+        default: return cudaErrorInvalidValue;
+        }
     }
+}
+
+// A unit's entry point.
+#define ALS_STAGE_ARGS int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s
+typedef cudaError_t (*StageLauncher)(ALS_STAGE_ARGS);
+
+// The unit that holds the kernels of `recon`.
+inline cudaError_t launch_stage_unit(const StageLauncher (&units)[kReconGroups], ALS_STAGE_ARGS) {
+    return units[recon_group(recon)](recon, flux, kind, shape, P, blocks_per_sm, s);
 }
 
 // Whole steps of `members` 1-D lines, one cluster of `blocks` blocks each.
@@ -259,12 +286,20 @@ void stage_tile_dim(int shape, int* tile) {
 // many as fit) sizes the persistent grid.  stage_tile_* report the tile of
 // a shape as the kernels of that unit were built, so the host always covers
 // the grid with the tiles the kernels expect.
-cudaError_t launch_stage_f64_1d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
-cudaError_t launch_stage_f64_2d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
-cudaError_t launch_stage_f64_3d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
-cudaError_t launch_stage_f32_1d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
-cudaError_t launch_stage_f32_2d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
-cudaError_t launch_stage_f32_3d(int recon, int flux, int kind, int shape, const StageParams& P, int blocks_per_sm, cudaStream_t s);
+cudaError_t launch_stage_f64_1d(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f64_2d(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f64_2d_eno(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f64_2d_limiter(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f64_3d(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f64_3d_eno(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f64_3d_limiter(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f32_1d(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f32_2d(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f32_2d_eno(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f32_2d_limiter(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f32_3d(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f32_3d_eno(ALS_STAGE_ARGS);
+cudaError_t launch_stage_f32_3d_limiter(ALS_STAGE_ARGS);
 cudaError_t launch_line_f64(int recon, int flux, bool rk3, const LineParams& P, int members, int blocks, cudaStream_t s);
 cudaError_t launch_line_f32(int recon, int flux, bool rk3, const LineParams& P, int members, int blocks, cudaStream_t s);
 void stage_tile_f64_1d(int shape, int* tile);

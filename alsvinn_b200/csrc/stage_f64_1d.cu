@@ -2,9 +2,10 @@
 #include "stage_dispatch.cuh"
 
 namespace als {
-cudaError_t launch_stage_f64_1d(int recon, int flux, int kind, int shape,
-    const StageParams& P, int blocks_per_sm, cudaStream_t s) {
-    return launch_stage_dim<double, 1>(recon, flux, kind, shape, P, blocks_per_sm, s);
+cudaError_t launch_stage_f64_1d(ALS_STAGE_ARGS) {
+    static const StageLauncher units[kReconGroups] = {launch_stage_group<double, 1, 0>,
+        launch_stage_group<double, 1, 1>, launch_stage_group<double, 1, 2>};
+    return launch_stage_unit(units, recon, flux, kind, shape, P, blocks_per_sm, s);
 }
 
 void stage_tile_f64_1d(int shape, int* tile) {

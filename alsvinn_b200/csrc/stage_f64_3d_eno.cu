@@ -1,0 +1,8 @@
+// Stage-kernel instantiations for double precision, 3-D Euler, the wide stencils (ENO3, ENO4, WENO3).
+#include "stage_dispatch.cuh"
+
+namespace als {
+cudaError_t launch_stage_f64_3d_eno(ALS_STAGE_ARGS) {
+    return launch_stage_group<double, 3, 1>(recon, flux, kind, shape, P, blocks_per_sm, s);
+}
+} // namespace als
