@@ -225,7 +225,8 @@ __host__ __device__ constexpr bool quick_face() {
     return sizeof(R) == 8 && (FLUX == FLUX_HLL || FLUX == FLUX_HLL3);
 }
 
-// face_flux with the straight-line form where there is one.
+// face_flux with the straight-line form where there is one, and FP32 with the
+// flushing reciprocals and roots where the face allows them.
 template<class R, int NSD, int FLUX, int D>
 __device__ __forceinline__ R face_flux_best(const R* ul, const R* ur, R gamma, R* F) {
     if constexpr (quick_face<R, FLUX>()) {
@@ -233,6 +234,11 @@ __device__ __forceinline__ R face_flux_best(const R* ul, const R* ur, R gamma, R
         face_quick<NSD, FLUX, D>(ul, ur, gamma, F, Q);
         face_settle<NSD, FLUX, D>(ul, ur, gamma, F, Q);
         return Q.w;
+    } else if constexpr (fast_recip<R>() && (FLUX == FLUX_HLL || FLUX == FLUX_HLL3)) {
+        FaceState<R, NSD> L, Rt;
+        make_state<R, NSD, D, true>(ul, gamma, L);
+        make_state<R, NSD, D, true>(ur, gamma, Rt);
+        return flux_between<R, NSD, FLUX, D, true>(L, Rt, gamma, F);
     } else {
         return face_flux<R, NSD, FLUX, D>(ul, ur, gamma, F);
     }

@@ -64,15 +64,15 @@ __host__ __device__ constexpr bool fast_recip() {
     return ALS_F32_RECIP != 0 && sizeof(R) == 4;
 }
 
-// Reciprocal and square root.  FP32 members take the hardware's approximations
-// in the form that flushes subnormals: the compiler's own forms test for them
-// and rescale, 110 of a cell and stage's 840 instructions (512 x 256^2 members,
-// ms per RK3 step: 2.70 -> 2.37).  Their operands are densities, sums of
-// squares above 1e-16, wave speeds and pressures over densities, so that only
-// values beyond 8e37 or below 1e-38 see the difference.
-template<class R>
+// Reciprocal and square root.  With FLUSH, FP32 takes the hardware's
+// approximations in the form that flushes subnormal operands and results to
+// zero: the compiler's own forms test for them and rescale, 110 of a cell and
+// stage's 840 instructions.  They are the same bits while operand and result
+// are normal; flush_applies tests the two states of a face for that, and a face
+// outside its range takes the plain forms.
+template<class R, bool FLUSH>
 __device__ __forceinline__ R recip(R x) {
-    if constexpr (fast_recip<R>()) {
+    if constexpr (fast_recip<R>() && FLUSH) {
         R y;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
         return y;
@@ -81,9 +81,9 @@ __device__ __forceinline__ R recip(R x) {
     }
 }
 
-template<class R>
+template<class R, bool FLUSH>
 __device__ __forceinline__ R root(R x) {
-    if constexpr (fast_recip<R>()) {
+    if constexpr (fast_recip<R>() && FLUSH) {
         R y;
         asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
         return y;
@@ -102,7 +102,7 @@ struct FaceState {
 };
 
 // computeExtra (Euler.hpp:204-211): ie = E - 0.5*(m.m)/rho, u = m/rho, p = (gamma-1)*ie.
-template<class R, int NSD, int D>
+template<class R, int NSD, int D, bool FLUSH>
 __device__ __forceinline__ void make_state(const R* U, R gamma, FaceState<R, NSD>& s) {
 #pragma unroll
     for (int k = 0; k < NSD + 2; ++k) {
@@ -116,7 +116,7 @@ __device__ __forceinline__ void make_state(const R* U, R gamma, FaceState<R, NSD
         dot = dot + U[3] * U[3];
     }
     if constexpr (fast_recip<R>()) {
-        const R ri = recip(U[0]);
+        const R ri = recip<R, FLUSH>(U[0]);
         s.ri = ri;
         s.ud = U[1 + D] * ri;
         s.p = (gamma - R(1)) * (U[NSD + 1] - R(0.5) * dot * ri);
@@ -137,6 +137,24 @@ __device__ __forceinline__ R sound2(const FaceState<R, NSD>& s, R gamma) {
     }
 }
 
+// Whether the FLUSH forms may take a face between two FP32 states: densities
+// and pressures in [2^-40, 2^40).  Why that suffices.  Sound speeds, and the Roe
+// value's, which lies between them, are at least 2^-40, and the roots of the
+// densities between 2^-20 and 2^20.  A pressure below 2^40 is left of an energy
+// below 2^(40 + 48 + 23) (a fused difference, gamma - 1 >= 2^-23), so velocities
+// are below 2^77 and rho (u - s) below 2^118.  A signal speed, a sum with a sound
+// speed in it, is 0 or at least 2^-64, and so is u - s; rho (u - s) of the two
+// sides have opposite signs, and 0 or the contact's speed lies between the
+// signal speeds, so their differences do not cancel below that (but for sR = 0,
+// which is sent to the plain form).  All reciprocals and roots then have normal
+// operands and results.  NaNs pass: they give NaN either way.
+template<class R, int NSD>
+__device__ __forceinline__ bool flush_applies(const FaceState<R, NSD>& L, const FaceState<R, NSD>& Rt) {
+    const R lo = fmin(fmin(L.c[0], Rt.c[0]), fmin(L.p, Rt.p));
+    const R hi = fmax(fmax(L.c[0], Rt.c[0]), fmax(L.p, Rt.p));
+    return lo >= R(9.094947017729282e-13) && hi < R(1099511627776.0);
+}
+
 // Point flux along D (Euler.hpp:172-181).
 template<class R, int NSD, int D>
 __device__ __forceinline__ void point_flux(const FaceState<R, NSD>& s, R* F) {
@@ -149,91 +167,96 @@ __device__ __forceinline__ void point_flux(const FaceState<R, NSD>& s, R* F) {
     F[NSD + 1] = (s.c[NSD + 1] + s.p) * s.ud;
 }
 
-template<class R, int NSD, int D>
+// The plain form of a face's flux, below.
+template<class R, int NSD, int FLUX, int D>
+__device__ __forceinline__ R face_flux(const R* ul, const R* ur, R gamma, R* F);
+
+// With FLUSH the common case, a star state in the range of the FLUSH forms, is
+// one test; a face outside it starts over.
+template<class R, int NSD, int D, bool FLUSH>
 __device__ __forceinline__ R flux_hll(const FaceState<R, NSD>& L, const FaceState<R, NSD>& Rt,
     R gamma, R* F) {
     constexpr int NV = NSD + 2;
-    const R wl = root(L.c[0]);
-    const R wr = root(Rt.c[0]);
+    const R wl = root<R, FLUSH>(L.c[0]);
+    const R wr = root<R, FLUSH>(Rt.c[0]);
     const R rho = (L.c[0] + Rt.c[0]) / R(2);
     R ud, p;
     if constexpr (fast_recip<R>()) {
-        const R iw = recip(wl + wr);
+        const R iw = recip<R, FLUSH>(wl + wr);
         ud = (wl * L.ud + wr * Rt.ud) * iw;
         p = (L.p * wl + Rt.p * wr) * iw;
     } else {
         ud = (wl * L.ud + wr * Rt.ud) / (wl + wr);
         p = (L.p * wl + Rt.p * wr) / (wl + wr);
     }
-    const R cs = root(fast_recip<R>() ? gamma * p * recip(rho) : gamma * p / rho);
-    const R sL = fmin(L.ud - root(sound2(L, gamma)), ud - cs);
-    const R sR = fmax(Rt.ud + root(sound2(Rt, gamma)), ud + cs);
-    if (sL == R(0)) {
+    const R cs = root<R, FLUSH>(fast_recip<R>() ? gamma * p * recip<R, FLUSH>(rho) : gamma * p / rho);
+    const R cl = root<R, FLUSH>(sound2(L, gamma));
+    const R cr = root<R, FLUSH>(sound2(Rt, gamma));
+    const R sL = fmin(L.ud - cl, ud - cs);
+    const R sR = fmax(Rt.ud + cr, ud + cs);
+    constexpr bool tested = fast_recip<R>() && FLUSH;
+    const bool inside = !tested || flush_applies(L, Rt);
+    if (inside && !(sL >= R(0)) && (tested ? !(sR <= R(0)) : !(sR < R(0)))) {
+        R FL[NV], FR[NV];
+        point_flux<R, NSD, D>(L, FL);
+        point_flux<R, NSD, D>(Rt, FR);
+        const R srsl = sR * sL;
+        const R den = sR - sL;
+        const R iden = fast_recip<R>() ? recip<R, FLUSH>(den) : R(0);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const R num = sR * FL[k] - sL * FR[k] + srsl * (Rt.c[k] - L.c[k]);
+            F[k] = fast_recip<R>() ? num * iden : num / den;
+        }
+    } else if (tested && (!inside || (sR == R(0) && !(sL >= R(0))))) {
+        return face_flux<R, NSD, FLUX_HLL, D>(L.c, Rt.c, gamma, F);
+    } else if (sL == R(0)) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             F[k] = R(0);
         }
     } else if (sL > R(0)) {
         point_flux<R, NSD, D>(L, F);
-    } else if (sR < R(0)) {
-        point_flux<R, NSD, D>(Rt, F);
     } else {
-        R FL[NV], FR[NV];
-        point_flux<R, NSD, D>(L, FL);
-        point_flux<R, NSD, D>(Rt, FR);
-        const R srsl = sR * sL;
-        const R den = sR - sL;
-        const R iden = fast_recip<R>() ? recip(den) : R(0);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            const R num = sR * FL[k] - sL * FR[k] + srsl * (Rt.c[k] - L.c[k]);
-            F[k] = fast_recip<R>() ? num * iden : num / den;
-        }
+        point_flux<R, NSD, D>(Rt, F);
     }
     return fmax(fabs(sL), fabs(sR));
 }
 
 // HLL3::computeHLLSpeeds (HLL3.hpp:120-160): Roe-averaged speeds with the
 // shock correction.
-template<class R, int NSD>
+template<class R, int NSD, bool FLUSH>
 __device__ __forceinline__ void hll3_speeds(const FaceState<R, NSD>& L, const FaceState<R, NSD>& Rt,
     R gamma, R& sL, R& sR) {
-    const R wl = root(L.c[0]);
-    const R wr = root(Rt.c[0]);
+    const R wl = root<R, FLUSH>(L.c[0]);
+    const R wr = root<R, FLUSH>(Rt.c[0]);
     const R rho = (L.c[0] + Rt.c[0]) / R(2);
     R ud, p;
     if constexpr (fast_recip<R>()) {
-        const R iw = recip(wl + wr);
+        const R iw = recip<R, FLUSH>(wl + wr);
         ud = (wl * L.ud + wr * Rt.ud) * iw;
         p = (wl * L.p + wr * Rt.p) * iw;
     } else {
         ud = (wl * L.ud + wr * Rt.ud) / (wl + wr);
         p = (wl * L.p + wr * Rt.p) / (wl + wr);
     }
-    const R cfL = root(sound2(L, gamma));
-    const R cfR = root(sound2(Rt, gamma));
+    const R cfL = root<R, FLUSH>(sound2(L, gamma));
+    const R cfR = root<R, FLUSH>(sound2(Rt, gamma));
     const R correct = R(0.5) * fmax(R(0), L.ud - Rt.ud);
-    const R cs = root(fast_recip<R>() ? gamma * p * recip(rho) : gamma * p / rho);
+    const R cs = root<R, FLUSH>(fast_recip<R>() ? gamma * p * recip<R, FLUSH>(rho) : gamma * p / rho);
     sL = fmin(L.ud + correct - cfL, ud - cs);
     sR = fmax(Rt.ud - correct + cfR, ud + cs);
 }
 
-template<class R, int NSD, int D>
+template<class R, int NSD, int D, bool FLUSH>
 __device__ __forceinline__ R flux_hll3(const FaceState<R, NSD>& L, const FaceState<R, NSD>& Rt,
     R gamma, R* F) {
     constexpr int NV = NSD + 2;
     R sL, sR;
-    hll3_speeds<R, NSD>(L, Rt, gamma, sL, sR);
-    if (sL == R(0)) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            F[k] = R(0);
-        }
-    } else if (sL > R(0)) {
-        point_flux<R, NSD, D>(L, F);
-    } else if (sR < R(0)) {
-        point_flux<R, NSD, D>(Rt, F);
-    } else {
+    hll3_speeds<R, NSD, FLUSH>(L, Rt, gamma, sL, sR);
+    constexpr bool tested = fast_recip<R>() && FLUSH;
+    const bool inside = !tested || flush_applies(L, Rt);
+    if (inside && !(sL >= R(0)) && (tested ? !(sR <= R(0)) : !(sR < R(0)))) {
         // Of the two point fluxes only the transverse momentum components
         // (c[1+k] * ud, k != D: Euler.hpp:172-181 adds p along D only) enter
         // before the star side is chosen; the chosen side's full point flux
@@ -243,7 +266,7 @@ __device__ __forceinline__ R flux_hll3(const FaceState<R, NSD>& L, const FaceSta
         const R udl = L.ud - sL;
         const R udr = Rt.ud - sR;
         const R aa = udr * Rt.c[0] - udl * L.c[0];
-        const R iaa = fast_recip<R>() ? recip(aa) : R(0);
+        const R iaa = fast_recip<R>() ? recip<R, FLUSH>(aa) : R(0);
         auto over_aa = [&](R x) { return fast_recip<R>() ? x * iaa : x / aa; };
         const R sm = over_aa(Rt.c[1 + D] * udr - L.c[1 + D] * udl + Rt.p - L.p);
         // us: transverse star velocities (the normal one is sm)
@@ -265,7 +288,7 @@ __device__ __forceinline__ R flux_hll3(const FaceState<R, NSD>& L, const FaceSta
         R FK[NV];
         point_flux<R, NSD, D>(S, FK);
         const R den = sm - sK;
-        const R iden = fast_recip<R>() ? recip(den) : R(0);
+        const R iden = fast_recip<R>() ? recip<R, FLUSH>(den) : R(0);
         auto over_den = [&](R x) { return fast_recip<R>() ? x * iden : x / den; };
         R mid[NV];
         mid[0] = over_den(S.c[0] * udk);
@@ -279,6 +302,17 @@ __device__ __forceinline__ R flux_hll3(const FaceState<R, NSD>& L, const FaceSta
         for (int k = 0; k < NV; ++k) {
             F[k] = FK[k] + sK * (mid[k] - S.c[k]);
         }
+    } else if (tested && (!inside || (sR == R(0) && !(sL >= R(0))))) {
+        return face_flux<R, NSD, FLUX_HLL3, D>(L.c, Rt.c, gamma, F);
+    } else if (sL == R(0)) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            F[k] = R(0);
+        }
+    } else if (sL > R(0)) {
+        point_flux<R, NSD, D>(L, F);
+    } else {
+        point_flux<R, NSD, D>(Rt, F);
     }
     return fmax(fabs(sL), fabs(sR));
 }
@@ -294,7 +328,7 @@ __device__ __forceinline__ R flux_central(const FaceState<R, NSD>& L, const Face
     for (int k = 0; k < NV; ++k) {
         F[k] = R(0.5) * (FL[k] + FR[k]);
     }
-    return fmax(fabs(L.ud) + root(sound2(L, gamma)), fabs(Rt.ud) + root(sound2(Rt, gamma)));
+    return fmax(fabs(L.ud) + sqrt(sound2(L, gamma)), fabs(Rt.ud) + sqrt(sound2(Rt, gamma)));
 }
 
 // Logarithmic mean (b - a) / (log b - log a), 0 when either difference is 0
@@ -376,27 +410,33 @@ __device__ __forceinline__ R flux_tecno1(const FaceState<R, NSD>& L, const FaceS
         F[NSD + 1] = R(1) / (R(2) * bar(0)) * e;
     }
     R sL, sR;
-    hll3_speeds<R, NSD>(L, Rt, gamma, sL, sR);
+    hll3_speeds<R, NSD, false>(L, Rt, gamma, sL, sR);
     return fmax(fabs(sL), fabs(sR));
 }
 
 // F(U-, U+) at one face along D.  ul = right-reconstructed value of the cell
 // left of the face, ur = left-reconstructed value of the cell to its right
 // (numflux_util.hpp:62-92).  Returns the face wave speed.
-template<class R, int NSD, int FLUX, int D>
-__device__ __forceinline__ R face_flux(const R* ul, const R* ur, R gamma, R* F) {
-    FaceState<R, NSD> L, Rt;
-    make_state<R, NSD, D>(ul, gamma, L);
-    make_state<R, NSD, D>(ur, gamma, Rt);
+template<class R, int NSD, int FLUX, int D, bool FLUSH>
+__device__ __forceinline__ R flux_between(const FaceState<R, NSD>& L, const FaceState<R, NSD>& Rt,
+    R gamma, R* F) {
     if (FLUX == FLUX_HLL) {
-        return flux_hll<R, NSD, D>(L, Rt, gamma, F);
+        return flux_hll<R, NSD, D, FLUSH>(L, Rt, gamma, F);
     } else if (FLUX == FLUX_HLL3) {
-        return flux_hll3<R, NSD, D>(L, Rt, gamma, F);
+        return flux_hll3<R, NSD, D, FLUSH>(L, Rt, gamma, F);
     } else if (FLUX == FLUX_TECNO1) {
         return flux_tecno1<R, NSD, D>(L, Rt, gamma, F);
     } else {
         return flux_central<R, NSD, D>(L, Rt, gamma, F);
     }
+}
+
+template<class R, int NSD, int FLUX, int D>
+__device__ __forceinline__ R face_flux(const R* ul, const R* ur, R gamma, R* F) {
+    FaceState<R, NSD> L, Rt;
+    make_state<R, NSD, D, false>(ul, gamma, L);
+    make_state<R, NSD, D, false>(ur, gamma, Rt);
+    return flux_between<R, NSD, FLUX, D, false>(L, Rt, gamma, F);
 }
 
 // ENO coefficients c[r][j] (ENOCoefficients.cpp:27-49), each the correctly
@@ -442,6 +482,16 @@ __device__ __forceinline__ R twice_reciprocal(R d, R recip) {
         out = R(2) / d;
     }
     return out;
+}
+
+// The factor of WENO2's smoothness denominators 3 (eps + b)^2.  The FP32
+// weights do not depend on a common factor of theirs, and a power of two
+// changes no rounding: with 2^-64 their sums are normal numbers, and so are
+// the reciprocals, for all b below 1e28 (neighbouring densities 1e14 apart;
+// without it the reciprocal is flushed from 2e9 on and the sum overflows at 3e9).
+template<class R>
+__host__ __device__ constexpr R weno2_scale() {
+    return fast_recip<R>() ? R(3) / R(18446744073709551616.0) : R(3);
 }
 
 // WENO2 weights (w0Left, w1Left, w0Right, w1Right) from the smoothness
@@ -595,15 +645,14 @@ __device__ __forceinline__ void reconstruct_d(const Fetch& f, R* left, R* right,
         const R dm = i0 - f.at(0, -1);
         const R b0 = dp * dp;
         const R b1 = dm * dm;
-        const R d0 = R(3) * (eps + b0) * (eps + b0);
-        const R d1 = R(3) * (eps + b1) * (eps + b1);
+        const R d0 = weno2_scale<R>() * (eps + b0) * (eps + b0);
+        const R d1 = weno2_scale<R>() * (eps + b1) * (eps + b1);
         R w0Left, w1Left, w0Right, w1Right;
         if constexpr (fast_recip<R>()) {
             // a0L = 1/d0, a1L = 2/d1, a0R = 2/d0, a1R = 1/d1 give w0L = d1/(d1 + 2 d0),
             // w1L = 2 d0/(d1 + 2 d0), w0R = 2 d1/(2 d1 + d0), w1R = d0/(2 d1 + d0)
-            // (d stays finite in FP32 while neighbouring densities differ by < 1e9)
-            const R rl = recip(d1 + R(2) * d0);
-            const R rr = recip(R(2) * d1 + d0);
+            const R rl = recip<R, true>(d1 + R(2) * d0);
+            const R rr = recip<R, true>(R(2) * d1 + d0);
             w0Left = d1 * rl;
             w1Left = R(2) * d0 * rl;
             w0Right = R(2) * d1 * rr;
@@ -687,15 +736,14 @@ __device__ __forceinline__ void reconstruct_d(const Fetch& f, R* left, R* right,
         const R dm = i0 - f.at(0, -1);
         const R b0 = dp * dp;
         const R b1 = dm * dm;
-        const R d0 = R(3) * (eps + b0) * (eps + b0);
-        const R d1 = R(3) * (eps + b1) * (eps + b1);
+        const R d0 = weno2_scale<R>() * (eps + b0) * (eps + b0);
+        const R d1 = weno2_scale<R>() * (eps + b1) * (eps + b1);
         R w0Left, w1Left, w0Right, w1Right;
         if constexpr (fast_recip<R>()) {
             // a0L = 1/d0, a1L = 2/d1, a0R = 2/d0, a1R = 1/d1 give w0L = d1/(d1 + 2 d0),
             // w1L = 2 d0/(d1 + 2 d0), w0R = 2 d1/(2 d1 + d0), w1R = d0/(2 d1 + d0)
-            // (d stays finite in FP32 while neighbouring densities differ by < 1e9)
-            const R rl = recip(d1 + R(2) * d0);
-            const R rr = recip(R(2) * d1 + d0);
+            const R rl = recip<R, true>(d1 + R(2) * d0);
+            const R rr = recip<R, true>(R(2) * d1 + d0);
             w0Left = d1 * rl;
             w1Left = R(2) * d0 * rl;
             w0Right = R(2) * d1 * rr;

@@ -344,8 +344,8 @@ __device__ __forceinline__ R stencil_face_flux(const R* src, int box, int S, R g
             ub[v] = src[v * box + b * S];
         }
         FaceState<R, NSD> A, B;
-        make_state<R, NSD, D>(ua, gamma, A);
-        make_state<R, NSD, D>(ub, gamma, B);
+        make_state<R, NSD, D, false>(ua, gamma, A);
+        make_state<R, NSD, D, false>(ub, gamma, B);
         w = fmax(w, flux_tecno1<R, NSD, D>(A, B, gamma, out));
     };
     R f01[NV], fm11[NV], f02[NV];
