@@ -64,6 +64,57 @@ __host__ __device__ constexpr bool fast_recip() {
     return ALS_F32_RECIP != 0 && sizeof(R) == 4;
 }
 
+// Sums and products with FP32's contraction written out.  FP32 multiplications
+// and additions may be contracted, and where a sum holds several products the
+// choice is the compiler's and depends on the code around it: a member's result
+// then depends on the kernel that its batch size selects, which WENO3, WENOF2
+// and the entropy-conservative flux showed.  a * b + c and c - a * b rounded once; the rest
+// rounded by itself.  FP64 rounds every operation.
+template<class R>
+__device__ __forceinline__ R mad_rn(R a, R b, R c) {
+    if constexpr (sizeof(R) == 4) {
+        return __fmaf_rn(a, b, c);
+    } else {
+        return a * b + c;
+    }
+}
+
+template<class R>
+__device__ __forceinline__ R nmad_rn(R a, R b, R c) {
+    if constexpr (sizeof(R) == 4) {
+        return __fmaf_rn(-a, b, c);
+    } else {
+        return c - a * b;
+    }
+}
+
+template<class R>
+__device__ __forceinline__ R mul_rn(R a, R b) {
+    if constexpr (sizeof(R) == 4) {
+        return __fmul_rn(a, b);
+    } else {
+        return a * b;
+    }
+}
+
+template<class R>
+__device__ __forceinline__ R add_rn(R a, R b) {
+    if constexpr (sizeof(R) == 4) {
+        return __fadd_rn(a, b);
+    } else {
+        return a + b;
+    }
+}
+
+template<class R>
+__device__ __forceinline__ R sub_rn(R a, R b) {
+    if constexpr (sizeof(R) == 4) {
+        return __fsub_rn(a, b);
+    } else {
+        return a - b;
+    }
+}
+
 // Reciprocal and square root.  With FLUSH, FP32 takes the hardware's
 // approximations in the form that flushes subnormal operands and results to
 // zero: the compiler's own forms test for them and rescale, 110 of a cell and
@@ -380,7 +431,13 @@ __device__ __forceinline__ R flux_tecno1(const FaceState<R, NSD>& L, const FaceS
         same = same && (L.c[k] == Rt.c[k]);
     }
     if (same) {
-        point_flux<R, NSD, D>(L, F);
+        // point_flux, contracted as written
+#pragma unroll
+        for (int k = 0; k < NSD; ++k) {
+            F[1 + k] = k == D ? mad_rn(L.c[1 + k], L.ud, L.p) : mul_rn(L.c[1 + k], L.ud);
+        }
+        F[0] = L.c[1 + D];
+        F[NSD + 1] = mul_rn(add_rn(L.c[NSD + 1], L.p), L.ud);
     } else if (NSD == 3 && D == 2) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
@@ -568,14 +625,14 @@ __device__ __forceinline__ void primitive_at(const Fetch& f, int o, R gamma, R& 
     R dot = f.at(1, o) * f.at(1, o);
 #pragma unroll
     for (int k = 1; k < NSD; ++k) {
-        dot = dot + f.at(1 + k, o) * f.at(1 + k, o);
+        dot = mad_rn(f.at(1 + k, o), f.at(1 + k, o), dot);
     }
 #pragma unroll
     for (int k = 0; k < NSD; ++k) {
         u[k] = f.at(1 + k, o) / rho;
     }
-    const R ie = f.at(NSD + 1, o) - R(0.5) * dot / rho;
-    p = (gamma - R(1)) * ie;
+    const R ie = sub_rn(f.at(NSD + 1, o), R(0.5) * dot / rho);
+    p = mul_rn(gamma - R(1), ie);
 }
 
 // One side of WENOF2 (WENOF2.hpp:70-121): the bounded primitive slope dP,
@@ -585,46 +642,46 @@ template<class R, int NSD, bool RIGHT>
 __device__ __forceinline__ void wenof2_side(R w0, R w1, R gamma, const R* rho, const R (*u)[NSD],
     const R* p, R* out) {
     const R BOUND = R(1.9);
-    R dr = w1 * (rho[1] - rho[0]) + w0 * (rho[2] - rho[1]);
+    R dr = mad_rn(w1, sub_rn(rho[1], rho[0]), w0 * sub_rn(rho[2], rho[1]));
     R du[NSD];
 #pragma unroll
     for (int k = 0; k < NSD; ++k) {
-        du[k] = w1 * (u[1][k] - u[0][k]) + w0 * (u[2][k] - u[1][k]);
+        du[k] = mad_rn(w1, sub_rn(u[1][k], u[0][k]), w0 * sub_rn(u[2][k], u[1][k]));
     }
-    R dp = w1 * (p[1] - p[0]) + w0 * (p[2] - p[1]);
+    R dp = mad_rn(w1, sub_rn(p[1], p[0]), w0 * sub_rn(p[2], p[1]));
     dr = fmax(-BOUND * rho[1], fmin(BOUND * rho[1], dr));
     dp = fmax(-BOUND * p[1], fmin(BOUND * p[1], dp));
     R dudu = du[0] * du[0];
     R umdu = u[1][0] * du[0];
 #pragma unroll
     for (int k = 1; k < NSD; ++k) {
-        dudu = dudu + du[k] * du[k];
-        umdu = umdu + u[1][k] * du[k];
+        dudu = mad_rn(du[k], du[k], dudu);
+        umdu = mad_rn(u[1][k], du[k], umdu);
     }
-    const R LL = R(0.125) * rho[1] * dudu - R(0.5) * fmin(R(0), dr * umdu) +
-        R(0.5) * dr * dr * dudu / rho[1];
+    const R LL = add_rn(nmad_rn(R(0.5), fmin(R(0), dr * umdu), R(0.125) * rho[1] * dudu),
+        R(0.5) * dr * dr * dudu / rho[1]);
     const R Rr = p[1] / (gamma - R(1));
     const R a = R(0.5) * sqrt(Rr / fmax(Rr, LL));
     R pr, pu[NSD], pp;
     if (RIGHT) {
-        pr = rho[1] + a * dr;
-        pp = p[1] + a * dp;
+        pr = mad_rn(a, dr, rho[1]);
+        pp = mad_rn(a, dp, p[1]);
     } else {
-        pr = rho[1] - a * dr;
-        pp = p[1] - a * dp;
+        pr = nmad_rn(a, dr, rho[1]);
+        pp = nmad_rn(a, dp, p[1]);
     }
     R dot = R(0);
 #pragma unroll
     for (int k = 0; k < NSD; ++k) {
-        pu[k] = RIGHT ? u[1][k] + a * du[k] : u[1][k] - a * du[k];
-        dot = k == 0 ? pu[0] * pu[0] : dot + pu[k] * pu[k];
+        pu[k] = RIGHT ? mad_rn(a, du[k], u[1][k]) : nmad_rn(a, du[k], u[1][k]);
+        dot = k == 0 ? pu[0] * pu[0] : mad_rn(pu[k], pu[k], dot);
     }
     out[0] = pr;
 #pragma unroll
     for (int k = 0; k < NSD; ++k) {
-        out[1 + k] = pu[k] * pr;
+        out[1 + k] = mul_rn(pu[k], pr);
     }
-    out[NSD + 1] = pp / (gamma - R(1)) + R(0.5) * pr * dot;
+    out[NSD + 1] = mad_rn(R(0.5) * pr, dot, pp / (gamma - R(1)));
 }
 
 // DEFER (FP64 WENO2 and WENOF2): `ok` false asks for a call without it.
@@ -684,22 +741,23 @@ __device__ __forceinline__ void reconstruct_d(const Fetch& f, R* left, R* right,
         const R v0 = f.at(0, -2), v1 = f.at(0, -1), v2 = f.at(0, 0), v3 = f.at(0, 1), v4 = f.at(0, 2);
         const R c1312 = R(13.0 / 12.0);
         const R quarter = R(1 / 4.0);
-        R q = v2 - R(2) * v3 + v4;
+        R q = add_rn(nmad_rn(R(2), v3, v2), v4);
         R beta0 = c1312 * (q * q);
-        q = R(3) * v2 - R(4) * v3 + v4;
-        beta0 = beta0 + quarter * (q * q);
-        q = v1 - R(2) * v2 + v3;
+        q = add_rn(nmad_rn(R(4), v3, R(3) * v2), v4);
+        beta0 = mad_rn(quarter, q * q, beta0);
+        q = add_rn(nmad_rn(R(2), v2, v1), v3);
         R beta1 = c1312 * (q * q);
-        q = v1 - v3;
-        beta1 = beta1 + quarter * (q * q);
-        q = v0 - R(2) * v1 + v2;
+        q = sub_rn(v1, v3);
+        beta1 = mad_rn(quarter, q * q, beta1);
+        q = add_rn(nmad_rn(R(2), v1, v0), v2);
         R beta2 = c1312 * (q * q);
-        q = v0 - R(4) * v1 + R(3) * v2;
-        beta2 = beta2 + quarter * (q * q);
+        q = mad_rn(R(3), v2, nmad_rn(R(4), v1, v0));
+        beta2 = mad_rn(quarter, q * q, beta2);
         const R cw0 = R(3.0 / 10.0), cw1 = R(3.0 / 5.0), cw2 = R(1.0 / 10.0);
-        const R d2 = (beta2 + eps) * (beta2 + eps);
-        const R d1 = (beta1 + eps) * (beta1 + eps);
-        const R d0 = (beta0 + eps) * (beta0 + eps);
+        const R e2 = add_rn(beta2, eps), e1 = add_rn(beta1, eps), e0 = add_rn(beta0, eps);
+        const R d2 = e2 * e2;
+        const R d1 = e1 * e1;
+        const R d0 = e0 * e0;
         R ar[3], al[3];
         ar[2] = cw2 / d2;
         al[2] = cw0 / d2;
@@ -718,11 +776,11 @@ __device__ __forceinline__ void reconstruct_d(const Fetch& f, R* left, R* right,
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
                     const R value = f.at(v, j - shift);
-                    lv += eno_coef<R, 3>(shift, j) * value;
-                    rv += eno_coef<R, 3>(shift + 1, j) * value;
+                    lv = mad_rn(eno_coef<R, 3>(shift, j), value, lv);
+                    rv = mad_rn(eno_coef<R, 3>(shift + 1, j), value, rv);
                 }
-                lw += lv * (al[shift] / sl);
-                rw += rv * (ar[shift] / sr);
+                lw = mad_rn(lv, al[shift] / sl, lw);
+                rw = mad_rn(rv, ar[shift] / sr, rw);
             }
             left[v] = lw;
             right[v] = rw;
