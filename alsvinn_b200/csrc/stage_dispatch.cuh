@@ -4,6 +4,9 @@
 // instantiations compile in parallel.
 #pragma once
 
+#include <algorithm>
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 #include "stage_faces.cuh"
@@ -14,15 +17,54 @@
 
 namespace als {
 
+// Blocks of KERNEL that the current device can hold at once.  A property of
+// the kernel and the device: looked up once per device.
+template<void (*KERNEL)(StageParams)>
+cudaError_t resident_blocks(int threads, size_t smem, int* blocks) {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];
+    int device = 0, sms = 0, per_sm = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) {
+        return err;
+    }
+    const bool kept = device >= 0 && device < kDevices;
+    if (kept && known[device].load(std::memory_order_relaxed) > 0) {
+        *blocks = known[device].load(std::memory_order_relaxed);
+        return cudaSuccess;
+    }
+    err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (err == cudaSuccess) {
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, threads, smem);
+    }
+    if (err != cudaSuccess) {
+        return err;
+    }
+    *blocks = (per_sm < 1 ? 1 : per_sm) * sms;
+    if (kept) {
+        known[device].store(*blocks, std::memory_order_relaxed);
+    }
+    return cudaSuccess;
+}
+
 // One block per work item when the launch has no work counter; otherwise a
 // persistent launch of as many blocks as can be resident at once (or
 // `blocks_per_sm` per SM when > 0, capped by what fits), never more than
 // there are work items.
-inline cudaError_t launch_stage_blocks(void (*kernel)(StageParams), int threads, size_t smem,
-    const StageParams& P, int blocks_per_sm, cudaStream_t stream) {
+//
+// The solver's stages may be chained: a stage's blocks take their places while
+// the one before it ends, which hides its launch (2 to 7 %).  Not with fewer
+// blocks than the GPU holds at once: the early ones then double up on the SMs
+// that the running stage leaves free, and the stage takes as long as those
+// (TeCNO6, 256^2, 128 tiles, us per RK3 step: 119 apart, 190 chained; KH 32^2 by
+// faces 17.9 and 20.2).  `small` kernels are chained all the same: bound by
+// latency, sharing an SM costs them nothing (FP32 faces, 64^2: 18.2 and 17.5).
+template<void (*KERNEL)(StageParams)>
+cudaError_t launch_stage_blocks(int threads, size_t smem, const StageParams& P, int blocks_per_sm,
+    cudaStream_t stream, bool small = false) {
     // raising the dynamic shared-memory limit is idempotent and cheap; it is
     // done on every launch so that every device the process uses is covered
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t err = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
         int(smem));
     if (err != cudaSuccess) {
         return err;
@@ -30,42 +72,37 @@ inline cudaError_t launch_stage_blocks(void (*kernel)(StageParams), int threads,
     if (P.total_work <= 0) {
         return cudaSuccess;
     }
+    int resident = 0;
+    if (P.counter || (P.chained && !small)) {
+        err = resident_blocks<KERNEL>(threads, smem, &resident);
+        if (err != cudaSuccess) {
+            return err;
+        }
+    }
+    long long blocks = P.total_work;
+    if (P.counter) {
+        int device = 0, sms = 0;
+        err = cudaGetDevice(&device);
+        if (err == cudaSuccess) {
+            err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        }
+        if (err != cudaSuccess) {
+            return err;
+        }
+        const long long wanted = blocks_per_sm > 0 ? (long long)blocks_per_sm * sms : resident;
+        blocks = std::min(blocks, std::min<long long>(resident, wanted));
+    }
     cudaLaunchAttribute chained;
     chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     chained.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(unsigned(P.total_work));
+    config.gridDim = dim3(unsigned(blocks));
     config.blockDim = dim3(unsigned(threads));
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     config.attrs = &chained;
-    config.numAttrs = P.chained ? 1 : 0;
-    if (!P.counter) {
-        return cudaLaunchKernelEx(&config, kernel, P);
-    }
-    int device = 0, sms = 0, resident = 0;
-    err = cudaGetDevice(&device);
-    if (err == cudaSuccess) {
-        err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    }
-    if (err == cudaSuccess) {
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
-    }
-    if (err != cudaSuccess) {
-        return err;
-    }
-    if (resident < 1) {
-        resident = 1;
-    }
-    if (blocks_per_sm > 0 && blocks_per_sm < resident) {
-        resident = blocks_per_sm;
-    }
-    long long blocks = (long long)resident * sms;
-    if (blocks > P.total_work) {
-        blocks = P.total_work;
-    }
-    config.gridDim = dim3(unsigned(blocks));
-    return cudaLaunchKernelEx(&config, kernel, P);
+    config.numAttrs = P.chained && (small || blocks >= resident) ? 1 : 0;
+    return cudaLaunchKernelEx(&config, KERNEL, P);
 }
 
 // The kernel of one (kernel id, kind): a thread per face for id kFacesKernel
@@ -76,19 +113,19 @@ template<class R, int DIM, int RECON, int FLUX, int KIND, int SHAPE>
 cudaError_t launch_stage_one(const StageParams& P, int b, cudaStream_t s) {
     if constexpr (SHAPE == kFacesKernel) {
         typedef FaceLayout<R, DIM, RECON, FLUX> Lay;
-        return launch_stage_blocks(faces_kernel<R, DIM, RECON, FLUX, KIND>, Lay::THREADS, Lay::SMEM,
-            P, b, s);
+        return launch_stage_blocks<faces_kernel<R, DIM, RECON, FLUX, KIND>>(Lay::THREADS, Lay::SMEM,
+            P, b, s, sizeof(R) == 4 && DIM < 3);
     } else if constexpr (SHAPE == kPlanesKernel) {
         typedef ZLayout<R, RECON, FLUX> Lay;
-        return launch_stage_blocks(zmarch_kernel<R, RECON, FLUX, KIND>, Lay::THREADS, Lay::SMEM, P,
+        return launch_stage_blocks<zmarch_kernel<R, RECON, FLUX, KIND>>(Lay::THREADS, Lay::SMEM, P,
             b, s);
     } else if constexpr (marches_rows(DIM, FLUX, SHAPE)) {
         typedef RowLayout<R, RECON, FLUX> Lay;
         // a block of the schedule stands for eight of these warps
-        return launch_stage_blocks(rows_kernel<R, RECON, FLUX, KIND>, 32, Lay::SMEM, P, 8 * b, s);
+        return launch_stage_blocks<rows_kernel<R, RECON, FLUX, KIND>>(32, Lay::SMEM, P, 8 * b, s);
     } else {
         typedef StageLayout<R, DIM, RECON, FLUX, SHAPE> Lay;
-        return launch_stage_blocks(stage_kernel<R, DIM, RECON, FLUX, KIND, SHAPE>, Lay::THREADS,
+        return launch_stage_blocks<stage_kernel<R, DIM, RECON, FLUX, KIND, SHAPE>>(Lay::THREADS,
             Lay::SMEM, P, b, s);
     }
 }
