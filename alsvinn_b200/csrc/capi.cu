@@ -170,32 +170,58 @@ long long region_cells(const als::GridDesc& gd) {
     return (long long)(gd.hi[0] - gd.lo[0]) * (gd.hi[1] - gd.lo[1]) * (gd.hi[2] - gd.lo[2]);
 }
 
-// Kernel for levels of tile shape `shape` with `cells` cells in all.  A thread
-// per face has the least latency but repeats work at its boxes' edges, so it
-// runs 1-D and the smallest grids; warps that march along y do the least work
-// but need long runs, so they run the largest; in 2-D the 16 x 16 tiles lie
-// between.  16 RK3 steps, WENO2 + HLL3, ms, thread per face / 16 x 16 tiles /
-// marching: FP64 192^2 0.51 / 0.62 / 0.85, 256^2 0.61 / 0.67 / 0.92, 288^2 0.77 /
-// 0.69 / 0.95, 512^2 2.01 / 1.27 / 1.40, 576^2 2.51 / 1.55 / 1.63; FP32 256^2
-// 0.40 / 0.48 / 0.64, 288^2 0.56 / 0.51 / 0.68, 512^2 1.41 / 0.87 / 0.88, 576^2
-// 1.75 / 1.04 / 0.90 (MC and ENO3 cross in the same places).  3-D, thread per
-// face / marching along z: FP64 32^3 1.00 / 1.42, 40^3 1.53 / 1.53, 48^3 2.33 /
-// 1.56; FP32 32^3 0.76 / 0.93, 48^3 1.74 / 0.99.
-constexpr long long kFacesCells2 = 72000;
+// Boxes of the thread-per-face kernel that cover the region of a grid.
+long long face_boxes(const als::GridDesc& gd, int dim, int precision) {
+    long long boxes = 1;
+    for (int d = 0; d < dim; ++d) {
+        const int t = tile_extent(precision, dim, d, als::kFacesKernel);
+        boxes *= (gd.hi[d] - gd.lo[d] + t - 1) / t;
+    }
+    return boxes;
+}
+
+// Kernel for levels of tile shape `shape` with `cells` cells in all, `boxes`
+// boxes of the thread-per-face kernel.  A thread per face has the least latency
+// but repeats work at its boxes' edges, so it runs the smallest grids, up to as
+// many boxes as the GPU takes in one or two rounds; warps that march along y (2-D)
+// and columns that march along z do the least work but need long runs, so they
+// run the largest; tiles and boxes lie between.
+//   1-D (a launch per stage; see line_blocks), WENO2 + HLL3, us per RK3 step, thread
+// per face / tiles of 256 cells: FP64 4096 lines of 64 cells 91 / 142, of 128 160 / 144,
+// of 256 235 / 152, of 1024 762 / 589; FP32 4096 of 256 107 / 98, of 1024 333 / 366.
+//   2-D (148 x 2 FP64, 148 x 4 FP32 boxes a round), thread per face / 16 x 16 tiles /
+// marching: FP64 192^2 (336 boxes) 31 / 35, 256^2 (592) 36 / 40 / 49, 288^2 (756) 47 /
+// 41 / 50, 512^2 123 / 77 / 80, 640^2 111 / 109 (tiles, marching); FP32 256^2 22 / 28 / 34,
+// 288^2 31 / 29 / 35, 512^2 83 / 51 / 45 (the other reconstructions and HLL cross in the
+// same places).  The central flux is too cheap for the repeated work in FP64: 128^2
+// (152) 18.7 / 23.8, 192^2 29.4 / 29.3, 256^2 32 / 31.  TeCNO1 has 32 x 16 tiles on the
+// larger grids (1024^2, FP64: 326, marching 388).
+//   3-D (148 boxes a round), thread per face / 8 x 8 x 4 boxes / marching: FP64, WENO2
+// 24^3 (144) 33 / 45 / 67, 28^3 (280) 47 / 51 / 76, 32^3 (352) 61 / 52 / 76, 48^3 146 / 79 /
+// 81; ENO3 24^3 34 / 45, 28^3 49 / 46 (face, boxes); FP32, WENO2 24^3 27 / 31 / 47, 28^3
+// 35 / 33 / 51, 40^3 71 / 35 / 53, 48^3 108 / 58 / 54.
 constexpr long long kTilesCells2[2] = {400000, 270000};   // FP64, FP32
-constexpr long long kFacesCells3 = 60000;
-int choose_kernel(int dim, int flux, int shape, long long cells, int precision) {
+constexpr long long kBoxesCells3 = 100000;
+int choose_kernel(int dim, int recon, int flux, int shape, int n0, long long cells, long long boxes,
+    int precision) {
     if (als::stencil_flux(flux) || (dim == 2 && shape != 0)) {
         return shape;
     }
-    if (dim == 1 || cells <= (dim == 2 ? kFacesCells2 : kFacesCells3)) {
+    const bool fp64 = precision == ALS_FP64;
+    if (dim == 1) {
+        // lines of at most 127 cells fill a box of faces, and half a tile
+        return boxes > 148 * 4 && n0 > 127 && (fp64 || n0 <= 512) ? 0 : als::kFacesKernel;
+    }
+    if (dim == 2) {
+        if (boxes <= (fp64 && flux == ALS_FLUX_CENTRAL ? 148 * 2 : 148 * 4)) {
+            return als::kFacesKernel;
+        }
+        return als::kernel_built(2, 0, flux, 1) && cells <= kTilesCells2[fp64 ? 0 : 1] ? 1 : 0;
+    }
+    if (boxes <= (fp64 && als::recon_ghosts(recon) <= 2 ? 148 * 2 : 148)) {
         return als::kFacesKernel;
     }
-    if (dim == 2 && als::kernel_built(2, 0, flux, 1) &&
-        cells <= kTilesCells2[precision == ALS_FP64 ? 0 : 1]) {
-        return 1;
-    }
-    return dim == 3 && shape == 1 ? als::kPlanesKernel : shape;
+    return shape == 1 && cells > kBoxesCells3 ? als::kPlanesKernel : 0;
 }
 
 // The tile shape a configuration starts on: in 3-D the columns marching along
@@ -209,8 +235,8 @@ int default_shape(int dim, int recon, int flux) {
 als::GridDesc plan_region(int dim, const int* n, int g, const int* lo, const int* hi, int recon,
     int flux, int members, int* kernel) {
     als::GridDesc gd = make_grid(dim, n, g, lo, hi);
-    *kernel = choose_kernel(dim, flux, default_shape(dim, recon, flux), region_cells(gd) * members,
-        ALS_FP64);
+    *kernel = choose_kernel(dim, recon, flux, default_shape(dim, recon, flux), gd.hi[0] - gd.lo[0],
+        region_cells(gd) * members, face_boxes(gd, dim, ALS_FP64) * members, ALS_FP64);
     gd = make_grid(dim, n, g, lo, hi, ALS_FP64, *kernel);
     if (als::marches_rows(dim, flux, *kernel)) {
         split_runs(gd, run_rows(strip_rows(gd) * members, ALS_FP64));
@@ -706,6 +732,7 @@ struct SolverLevel {
     als::GridDesc grid;           // tiles of this level's tile shape
     int shape = 0;                // its tile shape (stage_kernel.cuh)
     int kernel = 0;               // the kernel that runs its stages (plan_levels)
+    int line_blocks = 0;          // blocks per line when whole steps run in one launch (plan_lines)
     int first = 0;                // global index of its first member
     long long member_elems = 0;   // nvar * plane
     double dx[3];
@@ -727,6 +754,7 @@ struct als_solver {
     int members = 0;              // over all levels
     int subdomains = 0;           // 1: the members are subdomains of one grid (als_solver_decompose)
     int procs[3] = {1, 1, 1};     // subdomains per direction
+    bool lines = false;           // whole steps of 1-D lines in one launch (plan_lines)
     bool needs_state = false;     // split after its state was set: advancing waits for a new one
     int cur = 0;                  // RK2 ping-pong: 1 when U^n of active members sits in B
     als::StepState* state = nullptr;
@@ -927,20 +955,85 @@ int enqueue_step(als_solver* s, cudaEvent_t* ev = nullptr) {
     return ALS_OK;
 }
 
-// Whether whole steps of this solver run in one launch (stage_line.cuh):
-// 1-D RK2 / RK3 with a two-point flux and lines that fit a cluster's shared
-// memory.
-bool runs_lines(const als_solver* s) {
-    if (s->cfg.dimension != 1 || s->subdomains || s->cfg.flux > ALS_FLUX_CENTRAL ||
-        (s->cfg.integrator != ALS_INT_RK2 && s->cfg.integrator != ALS_INT_RK3)) {
-        return false;
+// Parameters of whole steps of a level's lines on `blocks` blocks each.
+als::LineParams line_params(const als_solver* s, const SolverLevel& L, int blocks) {
+    als::LineParams P;
+    std::memset(&P, 0, sizeof(P));
+    P.in = s->current(L);
+    P.even = s->current(L);
+    P.odd = s->cfg.integrator == ALS_INT_RK3 ? s->current(L) : s->other(L);
+    P.state = s->state + L.first;
+    P.plane = L.grid.plane;
+    P.n = L.grid.n[0];
+    P.ghosts = s->g;
+    P.bc = s->cfg.boundary;
+    P.gamma = s->cfg.gamma;
+    P.stride = (P.n + blocks - 1) / blocks + 2 * s->g;
+    return P;
+}
+
+// Blocks of the cluster that runs whole steps of one line of this level in one
+// launch (stage_line.cuh), 0 where a launch per stage is faster: the most blocks
+// with which all lines are resident at once, or the fewest a line fits on, in several
+// rounds, when that still pays.  It does for lines up to 127 cells (which leave half a tile
+// empty) and from 512 to 2048 (which fill a block's threads); between and beyond, up
+// to two rounds; the longest only side by side, and FP64 hardly.  us per RK3 step,
+// WENO2 + HLL3, clusters of 8 / 4 / 2 / 1 blocks and a launch per stage (MC, ENO4 and no
+// reconstruction cross in the same places, WENO3 on 1024 cells is 2 to 15 % slower in
+// several rounds):
+//   FP64 1024 cells, 1 line 7.4 / 8.4 / 11.5 / 19.2, 17.4; 64 lines 17 / 17 / 11.8 / 19.8,
+// 20.9; 148 lines 41 / 41 / 23 / 19.8, 28; 4096 lines -, -, 625 / 534, 589.  4096 lines of
+// 64 cells 56, 91; of 256 cells 222, 152; 296 of 256 cells 16.7, 24.  4096 cells: 1 line
+// 11.6, 16.2; 64 lines 39 (4), 43; 200 lines 134 (4), 112.  8192 cells: 1 line 19.7, 17.3;
+// 8 lines 19.9, 20.4; 64 lines 98, 75.
+//   FP32 1024 cells, 1 line 5.2, 13.7; 4096 lines 257, 333.  256 cells, 296 lines 10.8,
+// 18.3; 4096 lines 140, 98.  8192 cells, 8 lines 10.0, 17.3; 16 lines 19.4, 17.9.
+int line_blocks(const als_solver* s, const SolverLevel& L) {
+    const int n = L.grid.n[0];
+    const int members = L.cfg.members;
+    const bool fp64 = s->cfg.precision == ALS_FP64;
+    if (n > als::kLineBlocks * als::kLineCells || (fp64 && n > 4096 && members < 6)) {
+        return 0;
     }
-    for (const SolverLevel& L : s->levels) {
-        if (L.grid.n[0] > als::kLineBlocks * als::kLineCells) {
-            return false;
+    const int most_rounds = n <= 128 || (n >= 512 && n <= 2048) ? INT_MAX : (n <= 4096 ? 2 : 1);
+    int fewest = 0, rounds = 0;
+    for (int blocks = als::kLineBlocks; blocks >= 1; blocks /= 2) {
+        // pieces of 64 cells or more, which also covers any stencil, and at most
+        // what the shared memory holds
+        if ((blocks > 1 && n / blocks < 64) || (n + blocks - 1) / blocks > als::kLineCells) {
+            continue;
         }
+        int clusters = 0;
+        const als::LineParams P = line_params(s, L, blocks);
+        if ((fp64 ? als::launch_line_f64 : als::launch_line_f32)(s->cfg.reconstruction, s->cfg.flux,
+                s->cfg.integrator == ALS_INT_RK3, P, members, blocks, s->stream, &clusters) !=
+                cudaSuccess || clusters < 1) {
+            cudaGetLastError();   // not a launch of its own: left to the stages
+            continue;
+        }
+        if (clusters >= members) {
+            return blocks;
+        }
+        fewest = blocks;
+        rounds = (members + clusters - 1) / clusters;
     }
-    return true;
+    return fewest > 0 && rounds <= most_rounds ? fewest : 0;
+}
+
+// Whether whole steps of this solver run in one launch: 1-D RK2 / RK3 with a
+// two-point flux, where every level chooses it.
+void plan_lines(als_solver* s) {
+    bool lines = s->cfg.dimension == 1 && s->cfg.flux <= ALS_FLUX_CENTRAL &&
+        (s->cfg.integrator == ALS_INT_RK2 || s->cfg.integrator == ALS_INT_RK3);
+    for (SolverLevel& L : s->levels) {
+        L.line_blocks = lines ? line_blocks(s, L) : 0;
+        lines = lines && L.line_blocks > 0;
+    }
+    s->lines = lines;
+}
+
+bool runs_lines(const als_solver* s) {
+    return s->lines && !s->subdomains;
 }
 
 // Enqueues `steps` time steps of every line, at most kLineSteps per launch
@@ -951,26 +1044,11 @@ int enqueue_lines(als_solver* s, long long steps) {
     while (steps > 0) {
         const int count = int(std::min(steps, kLineSteps));
         for (const SolverLevel& L : s->levels) {
-            als::LineParams P;
-            std::memset(&P, 0, sizeof(P));
-            P.in = s->current(L);
-            P.even = s->current(L);
-            P.odd = rk3 ? s->current(L) : s->other(L);
-            P.state = s->state + L.first;
-            P.plane = L.grid.plane;
-            P.n = L.grid.n[0];
-            P.ghosts = s->g;
-            P.bc = s->cfg.boundary;
+            als::LineParams P = line_params(s, L, L.line_blocks);
             P.steps = count;
-            P.gamma = s->cfg.gamma;
-            // pieces of 64 cells or more, which also covers any stencil
-            int blocks = als::kLineBlocks;
-            while (blocks > 1 && P.n / blocks < 64) {
-                blocks /= 2;
-            }
-            P.stride = (P.n + blocks - 1) / blocks + 2 * s->g;
             ALS_CUDA((s->cfg.precision == ALS_FP64 ? als::launch_line_f64 : als::launch_line_f32)(
-                s->cfg.reconstruction, s->cfg.flux, rk3, P, L.cfg.members, blocks, s->stream));
+                s->cfg.reconstruction, s->cfg.flux, rk3, P, L.cfg.members, L.line_blocks, s->stream,
+                nullptr));
         }
         if (!rk3) {
             s->cur ^= count & 1;
@@ -1045,11 +1123,15 @@ void plan_levels(als_solver* s) {
     const int dim = s->cfg.dimension;
     int lo[3] = {0, 0, 0};
     for (SolverLevel& L : s->levels) {
-        long long cells = 0;
+        long long cells = 0, boxes = 0;
         for (const SolverLevel& M : s->levels) {
-            cells += M.shape == L.shape ? region_cells(M.grid) * M.cfg.members : 0;
+            if (M.shape == L.shape) {
+                cells += region_cells(M.grid) * M.cfg.members;
+                boxes += face_boxes(M.grid, dim, s->cfg.precision) * M.cfg.members;
+            }
         }
-        L.kernel = choose_kernel(dim, s->cfg.flux, L.shape, cells, s->cfg.precision);
+        L.kernel = choose_kernel(dim, s->cfg.reconstruction, s->cfg.flux, L.shape, L.grid.n[0], cells,
+            boxes, s->cfg.precision);
         L.grid = make_grid(dim, L.grid.n, s->g, lo, L.grid.n, s->cfg.precision, L.kernel);
     }
     long long rows = 0, planes = 0;
@@ -1189,6 +1271,7 @@ int als_solver_create_levels(const als_solver_config* cfgs, int nlevels, int dev
         s->levels.push_back(L);
     }
     plan_levels(s.get());
+    plan_lines(s.get());
     s->members = first;
     s->order.resize(nlevels);
     std::iota(s->order.begin(), s->order.end(), 0);

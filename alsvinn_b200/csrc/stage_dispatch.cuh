@@ -233,9 +233,12 @@ inline cudaError_t launch_stage_unit(const StageLauncher (&units)[kReconGroups],
     return units[recon_group(recon)](recon, flux, kind, shape, P, blocks_per_sm, s);
 }
 
-// Whole steps of `members` 1-D lines, one cluster of `blocks` blocks each.
+// Whole steps of `members` 1-D lines, one cluster of `blocks` blocks each; with
+// `clusters` only the number of clusters that can be resident at once.
+#define ALS_LINE_ARGS bool rk3, const LineParams& P, int members, int blocks, cudaStream_t s, int* clusters
 template<class R, int RECON, int FLUX, bool RK3>
-cudaError_t launch_line_one(const LineParams& P, int members, int blocks, cudaStream_t stream) {
+cudaError_t launch_line_one(const LineParams& P, int members, int blocks, cudaStream_t stream,
+    int* clusters) {
     auto kernel = line_kernel<R, RECON, FLUX, RK3>;
     const size_t smem = LineLayout<R, RECON, FLUX>::smem(P.stride);
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -258,33 +261,38 @@ cudaError_t launch_line_one(const LineParams& P, int members, int blocks, cudaSt
     config.stream = stream;
     config.attrs = &cluster;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, P);
+    return clusters ? cudaOccupancyMaxActiveClusters(clusters, kernel, &config)
+                    : cudaLaunchKernelEx(&config, kernel, P);
+}
+
+template<class R, int RECON, int FLUX>
+cudaError_t launch_line_steps(ALS_LINE_ARGS) {
+    return rk3 ? launch_line_one<R, RECON, FLUX, true>(P, members, blocks, s, clusters)
+               : launch_line_one<R, RECON, FLUX, false>(P, members, blocks, s, clusters);
 }
 
 template<class R, int RECON>
-cudaError_t launch_line_flux(int flux, bool rk3, const LineParams& P, int members, int blocks,
-    cudaStream_t s) {
+cudaError_t launch_line_flux(int flux, ALS_LINE_ARGS) {
     switch (flux) {
-    case FLUX_HLL: return rk3 ? launch_line_one<R, RECON, FLUX_HLL, true>(P, members, blocks, s) : launch_line_one<R, RECON, FLUX_HLL, false>(P, members, blocks, s);
-    case FLUX_HLL3: return rk3 ? launch_line_one<R, RECON, FLUX_HLL3, true>(P, members, blocks, s) : launch_line_one<R, RECON, FLUX_HLL3, false>(P, members, blocks, s);
-    case FLUX_CENTRAL: return rk3 ? launch_line_one<R, RECON, FLUX_CENTRAL, true>(P, members, blocks, s) : launch_line_one<R, RECON, FLUX_CENTRAL, false>(P, members, blocks, s);
+    case FLUX_HLL: return launch_line_steps<R, RECON, FLUX_HLL>(rk3, P, members, blocks, s, clusters);
+    case FLUX_HLL3: return launch_line_steps<R, RECON, FLUX_HLL3>(rk3, P, members, blocks, s, clusters);
+    case FLUX_CENTRAL: return launch_line_steps<R, RECON, FLUX_CENTRAL>(rk3, P, members, blocks, s, clusters);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template<class R>
-cudaError_t launch_line(int recon, int flux, bool rk3, const LineParams& P, int members,
-    int blocks, cudaStream_t s) {
+cudaError_t launch_line(int recon, int flux, ALS_LINE_ARGS) {
     switch (recon) {
-    case RECON_NONE: return launch_line_flux<R, RECON_NONE>(flux, rk3, P, members, blocks, s);
-    case RECON_WENO2: return launch_line_flux<R, RECON_WENO2>(flux, rk3, P, members, blocks, s);
-    case RECON_ENO2: return launch_line_flux<R, RECON_ENO2>(flux, rk3, P, members, blocks, s);
-    case RECON_ENO3: return launch_line_flux<R, RECON_ENO3>(flux, rk3, P, members, blocks, s);
-    case RECON_ENO4: return launch_line_flux<R, RECON_ENO4>(flux, rk3, P, members, blocks, s);
-    case RECON_MC: return launch_line_flux<R, RECON_MC>(flux, rk3, P, members, blocks, s);
-    case RECON_MM: return launch_line_flux<R, RECON_MM>(flux, rk3, P, members, blocks, s);
-    case RECON_WENOF2: return launch_line_flux<R, RECON_WENOF2>(flux, rk3, P, members, blocks, s);
-    case RECON_WENO3: return launch_line_flux<R, RECON_WENO3>(flux, rk3, P, members, blocks, s);
+    case RECON_NONE: return launch_line_flux<R, RECON_NONE>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_WENO2: return launch_line_flux<R, RECON_WENO2>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_ENO2: return launch_line_flux<R, RECON_ENO2>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_ENO3: return launch_line_flux<R, RECON_ENO3>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_ENO4: return launch_line_flux<R, RECON_ENO4>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_MC: return launch_line_flux<R, RECON_MC>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_MM: return launch_line_flux<R, RECON_MM>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_WENOF2: return launch_line_flux<R, RECON_WENOF2>(flux, rk3, P, members, blocks, s, clusters);
+    case RECON_WENO3: return launch_line_flux<R, RECON_WENO3>(flux, rk3, P, members, blocks, s, clusters);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -337,8 +345,8 @@ cudaError_t launch_stage_f32_2d_limiter(ALS_STAGE_ARGS);
 cudaError_t launch_stage_f32_3d(ALS_STAGE_ARGS);
 cudaError_t launch_stage_f32_3d_eno(ALS_STAGE_ARGS);
 cudaError_t launch_stage_f32_3d_limiter(ALS_STAGE_ARGS);
-cudaError_t launch_line_f64(int recon, int flux, bool rk3, const LineParams& P, int members, int blocks, cudaStream_t s);
-cudaError_t launch_line_f32(int recon, int flux, bool rk3, const LineParams& P, int members, int blocks, cudaStream_t s);
+cudaError_t launch_line_f64(int recon, int flux, ALS_LINE_ARGS);
+cudaError_t launch_line_f32(int recon, int flux, ALS_LINE_ARGS);
 void stage_tile_f64_1d(int shape, int* tile);
 void stage_tile_f64_2d(int shape, int* tile);
 void stage_tile_f64_3d(int shape, int* tile);

@@ -11,9 +11,8 @@ cudaError_t launch_stage_f32_1d(ALS_STAGE_ARGS) {
 void stage_tile_f32_1d(int shape, int* tile) {
     stage_tile_dim<1>(shape, tile);
 }
-cudaError_t launch_line_f32(int recon, int flux, bool rk3, const LineParams& P, int members,
-    int blocks, cudaStream_t s) {
-    return launch_line<float>(recon, flux, rk3, P, members, blocks, s);
-}
 
+cudaError_t launch_line_f32(int recon, int flux, ALS_LINE_ARGS) {
+    return launch_line<float>(recon, flux, rk3, P, members, blocks, s, clusters);
+}
 } // namespace als

@@ -156,7 +156,7 @@ constexpr int kFacesKernel = 2;
 constexpr int kPlanesKernel = 3;
 constexpr int kMaxKernels = 4;
 
-// Two-point fluxes have it in every dimension; in 1-D it is the only one.  In
+// Two-point fluxes have it in every dimension.  In
 // 2-D the 16 x 16 tiles also serve levels of shape 0 (als_solver_set_tiles
 // offers shape 1 where shape_built says), so they are built for every
 // reconstruction.
@@ -165,12 +165,12 @@ __host__ __device__ constexpr bool kernel_built(int dim, int recon, int flux, in
         : kernel == kPlanesKernel ? dim == 3 && shape_built(dim, recon, flux, 1)
         : dim == 3 && kernel == 1 ? false
         : (dim == 2 && kernel == 1 && flux <= FLUX_CENTRAL) ||
-            (shape_built(dim, recon, flux, kernel) && (dim > 1 || stencil_flux(flux)));
+            shape_built(dim, recon, flux, kernel);
 }
 
 // Whether a kernel's work items are runs of rows (stage_rows.cuh).
 __host__ __device__ constexpr bool marches_rows(int dim, int flux, int kernel) {
-    return dim == 2 && kernel == 0 && !stencil_flux(flux);
+    return dim == 2 && kernel == 0 && flux <= FLUX_CENTRAL;
 }
 
 // Whether they are segments of planes (stage_zmarch.cuh).

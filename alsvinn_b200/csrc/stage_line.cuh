@@ -38,7 +38,7 @@ struct LineParams {
     double gamma;
 };
 
-constexpr int kLineThreads = 256;     // most threads of a block
+constexpr int kLineThreads = 288;     // most threads of a block: the 257 faces of 256 cells in one pass
 constexpr int kLineBlocks = 8;        // blocks per cluster, at most (the portable size)
 constexpr int kLineCells = 1024;      // cells of a block's piece, at most
 
