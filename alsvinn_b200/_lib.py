@@ -109,6 +109,7 @@ PROTOTYPES = {
     "als_solver_synchronize": (ctypes.c_int, [_VP]),
     "als_solver_stream": (_VP, [_VP]),
     "als_solver_launches_per_step": (ctypes.c_int, [_VP]),
+    "als_solver_get_kernels": (ctypes.c_int, [_VP, _I]),
     "als_solver_profile_step": (ctypes.c_int, [_VP, ctypes.POINTER(ctypes.c_float), ctypes.c_int]),
     "als_uniform_draws": (ctypes.c_int, [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong,
                                          ctypes.c_double, ctypes.c_double, _D]),

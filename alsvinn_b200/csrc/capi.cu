@@ -1677,21 +1677,47 @@ int als_solver_launches_per_step(const als_solver* s) {
     if (!s) {
         return fail(ALS_E_INVALID, "null solver");
     }
-    if (s->cfg.integrator == ALS_INT_RK3) {
-        return 3;
+    const int levels = int(s->levels.size());
+    if (runs_lines(s)) {
+        return levels;
     }
-    if (s->cfg.integrator == ALS_INT_RK2) {
-        return 2;
+    // levels that one kernel runs share a stage's launch
+    std::vector<int> kernels;
+    for (const SolverLevel& L : s->levels) {
+        kernels.push_back(L.kernel);
     }
-    return 1 + int(s->levels.size());
+    std::sort(kernels.begin(), kernels.end());
+    const int launches = int(std::unique(kernels.begin(), kernels.end()) - kernels.begin());
+    switch (s->cfg.integrator) {
+    case ALS_INT_RK3: return 3 * launches;
+    case ALS_INT_RK2: return 2 * launches;
+    default: return launches + levels;   // forward Euler updates level by level
+    }
+}
+
+int als_solver_get_kernels(const als_solver* s, int* kernels) {
+    if (!s || !kernels) {
+        return fail(ALS_E_INVALID, "null argument");
+    }
+    for (size_t l = 0; l < s->levels.size(); ++l) {
+        const int k = s->levels[l].kernel;
+        kernels[l] = runs_lines(s) ? ALS_KERNEL_LINES
+            : als::marches_rows(s->cfg.dimension, s->cfg.flux, k) ? ALS_KERNEL_ROWS
+            : k == als::kFacesKernel ? ALS_KERNEL_FACES
+            : k == als::kPlanesKernel ? ALS_KERNEL_COLUMNS
+            : k == 1 ? ALS_KERNEL_SMALL_TILES : ALS_KERNEL_TILES;
+    }
+    return ALS_OK;
 }
 
 int als_solver_profile_step(als_solver* s, float* kernel_ms, int capacity) {
     if (!s || !kernel_ms) {
         return fail(ALS_E_INVALID, "null argument");
     }
-    // events sit between the stages: FE counts its per-level updates as one
-    const int k = s->cfg.integrator == ALS_INT_RK3 ? 3 : 2;
+    // events sit between the stages: FE counts its per-level updates as one,
+    // and whole steps in one launch (lines) are one
+    const bool lines = runs_lines(s);
+    const int k = lines ? 1 : (s->cfg.integrator == ALS_INT_RK3 ? 3 : 2);
     if (capacity < k) {
         return fail(ALS_E_INVALID, "capacity below the stages per step");
     }
@@ -1703,7 +1729,13 @@ int als_solver_profile_step(als_solver* s, float* kernel_ms, int capacity) {
             rc = fail(ALS_E_CUDA, "cudaEventCreate failed");
         }
     }
-    if (rc == ALS_OK) {
+    if (rc == ALS_OK && lines) {
+        rc = cudaEventRecord(ev[0], s->stream) == cudaSuccess ? enqueue_lines(s, 1)
+                                                              : fail(ALS_E_CUDA, "cudaEventRecord failed");
+        if (rc == ALS_OK && cudaEventRecord(ev[1], s->stream) != cudaSuccess) {
+            rc = fail(ALS_E_CUDA, "cudaEventRecord failed");
+        }
+    } else if (rc == ALS_OK) {
         rc = enqueue_step(s, ev);
     }
     if (rc == ALS_OK && cudaEventSynchronize(ev[k]) != cudaSuccess) {
@@ -1801,7 +1833,8 @@ int als_solver_get_tiles(const als_solver* s, int* tile_shapes, int* tile_extent
 // same saved state, keeps the fastest, and restores the state and member
 // clocks, so tuning changes no result.  First the tile shape of each level
 // (coordinate search: one level's shape varied at a time, the others at
-// their best so far), then persistent blocks per SM x level order.
+// their best so far), then persistent blocks per SM x level order.  Lines whose
+// whole steps run in one launch have no schedule: they are timed as they run.
 int als_solver_tune(als_solver* s, int steps, int* blocks_per_sm, int* level_order,
     int* tile_shapes, double* best_ms_per_step) {
     if (!s || steps < 1) {
@@ -1874,6 +1907,7 @@ int als_solver_tune(als_solver* s, int steps, int* blocks_per_sm, int* level_ord
     ALS_CUDA(cudaEventCreate(&e0));
     ALS_CUDA(cudaEventCreate(&e1));
     int rc = ALS_OK;
+    const bool lines = runs_lines(s);
     // ms per step of the current shapes, order and blocks per SM (1e300 after an error)
     auto time_steps = [&]() -> double {
         if (rc != ALS_OK) {
@@ -1885,8 +1919,10 @@ int als_solver_tune(als_solver* s, int steps, int* blocks_per_sm, int* level_ord
             if (k == 1 && cudaEventRecord(e0, s->stream) != cudaSuccess) {
                 rc = fail(ALS_E_CUDA, "cudaEventRecord failed");
             }
-            if (rc == ALS_OK) {
+            if (rc == ALS_OK && !lines) {
                 rc = enqueue_step(s);
+            } else if (rc == ALS_OK && k < 2) {
+                rc = enqueue_lines(s, k == 0 ? 1 : steps);
             }
         }
         if (rc == ALS_OK && (cudaEventRecord(e1, s->stream) != cudaSuccess ||
@@ -1923,7 +1959,7 @@ int als_solver_tune(als_solver* s, int steps, int* blocks_per_sm, int* level_ord
     std::vector<int> best_order = order0;
     for (const std::vector<int>& ord : orders) {
         for (int bps : bps_candidates) {
-            if (rc != ALS_OK) {
+            if (rc != ALS_OK || lines) {
                 break;
             }
             if (ord == order0 && bps == bps0) {

@@ -22,6 +22,7 @@ RECONSTRUCTION = {"none": 0, "weno2": 1, "eno2": 2, "eno3": 3, "eno4": 4, "mc": 
 INTEGRATOR = {"forwardeuler": 0, "rungekutta2": 1, "rungekutta3": 2, "rungekutta4": 3}
 BOUNDARY = {"neumann": 0, "periodic": 1}
 PRECISION = {"fp64": 0, "fp32": 1}
+KERNELS = ("tiles", "small tiles", "faces", "columns", "rows", "lines")
 EQUATION = {"euler1": 1, "euler2": 2, "euler3": 3}
 
 _D = ctypes.POINTER(ctypes.c_double)
@@ -185,10 +186,19 @@ class Simulator:
                 "status": info.status, "bad_index": info.bad_index, "bad_step": info.bad_step}
 
     def launches_per_step(self):
+        """Launches of one step advanced by itself (lines: one per level, which
+        covers up to 2,048 steps advanced together)."""
         return _lib.check(self._lib.als_solver_launches_per_step(self._h))
 
+    def kernels(self):
+        """The kernel that runs each level, chosen by its size and scheme."""
+        out = (ctypes.c_int * len(self.levels))()
+        _lib.check(self._lib.als_solver_get_kernels(self._h, out))
+        return [KERNELS[k] for k in out]
+
     def profile_step(self):
-        """Runs one step with events between the stages; returns their durations in ms."""
+        """Runs one step with events between the stages; returns their durations
+        in ms (lines: the one of the whole step)."""
         buf = (ctypes.c_float * 8)()
         k = _lib.check(self._lib.als_solver_profile_step(self._h, buf, 8))
         return [buf[i] for i in range(k)]

@@ -250,12 +250,22 @@ int als_solver_info(als_solver* s, int member, als_member_info* info);
 int als_solver_synchronize(als_solver* s);
 /* the stream the solver enqueues on (a cudaStream_t) */
 void* als_solver_stream(als_solver* s);
-/* Kernel launches a single time step issues (for launch accounting). */
+/* Kernel launches a single time step issues (for launch accounting): one per
+ * stage and kernel that the levels run on.  Lines (ALS_KERNEL_LINES): one per
+ * level, which covers up to 2,048 steps when they are advanced together. */
 int als_solver_launches_per_step(const als_solver* s);
-/* Runs one time step with CUDA events around each kernel (the reference's
+/* The kernel that runs each level, as its size and scheme choose it. */
+enum { ALS_KERNEL_TILES = 0,       /* box tiles (32x16, 8x8x4, 256 cells) */
+       ALS_KERNEL_SMALL_TILES = 1, /* 2-D 16x16 tiles */
+       ALS_KERNEL_FACES = 2,       /* a thread per face */
+       ALS_KERNEL_COLUMNS = 3,     /* 3-D, marching along z */
+       ALS_KERNEL_ROWS = 4,        /* 2-D, marching along y */
+       ALS_KERNEL_LINES = 5 };     /* 1-D, whole steps in one launch */
+int als_solver_get_kernels(const als_solver* s, int* kernels);
+/* Runs one time step with CUDA events around each stage (the reference's
  * ALSVINN_TIME_CUDA_BLOCK, alsutils/include/alsutils/timer/CudaTimer.hpp:42-47);
- * kernel_ms[k] receives the duration of kernel k.  Synchronises; returns the
- * number of kernels. */
+ * kernel_ms[k] receives the duration of stage k (lines: of the whole step, their
+ * one launch).  Synchronises; returns the number of durations. */
 int als_solver_profile_step(als_solver* s, float* kernel_ms, int capacity);
 /* Schedule of the stage launches: blocks_per_sm = 0 launches one block per
  * work item (level, member, tile); k > 0 makes every stage one persistent
@@ -280,8 +290,8 @@ int als_solver_get_tiles(const als_solver* s, int* tile_shapes, int* tile_extent
  * are unchanged.  It searches the tile shape of each level first (one level
  * varied at a time, the others at their best so far), then blocks per SM in
  * {0 (one per item), 1, 2, 3, 4} x level order in {as created, finest
- * first, coarsest first}.  Returns the choice (any out pointer may be NULL)
- * and its ms per step.  This replaces the reference's serial sample loop
+ * first, coarsest first}.  Lines have nothing to choose.  Returns the choice (any
+ * out pointer may be NULL) and its ms per step.  This replaces the reference's serial sample loop
  * (alsuq/src/run/Runner.cpp:42-78), which has no schedule to choose. */
 int als_solver_tune(als_solver* s, int steps, int* blocks_per_sm, int* level_order,
     int* tile_shapes, double* best_ms_per_step);
