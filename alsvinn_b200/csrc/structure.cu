@@ -55,6 +55,7 @@ struct StructGeom {
     long long plane;
     int tile[3];    // cells per block and direction
     int tiles[3];
+    bool staged;    // the cube statistic from a staged box
 };
 
 // FastPower<p> (alsutils/math/FastPower.hpp) for p = 1..5, pow otherwise
@@ -377,9 +378,24 @@ __global__ void structure_finish(const double* __restrict__ partial, int tiles, 
          t += (long long)gridDim.x * blockDim.x) {
         const long long r = t / H;
         const int h = int(t - r * H);
+        const double* p = partial + r * tiles * H + h;
         double s = 0;
-        for (int b = 0; b < tiles; ++b) {
-            s += partial[(r * tiles + b) * H + h];
+        int b = 0;
+        // sixteen loads in flight: one after another they took longer than the
+        // differences (128 x 128, H = 2, one state: 46 -> 34 us)
+        for (; b + 16 <= tiles; b += 16) {
+            double v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                v[k] = p[(long long)(b + k) * H];
+            }
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                s += v[k];
+            }
+        }
+        for (; b < tiles; ++b) {
+            s += p[(long long)b * H];
         }
         out[t] = s / cells;
     }
@@ -391,7 +407,24 @@ constexpr int kCubeH2 = 8;
 constexpr int kCubeH3 = 6;
 
 __host__ __device__ constexpr bool staged_cube(int dim, bool cube, int H) {
-    return cube && ((dim == 2 && H <= kCubeH2) || (dim == 3 && H <= kCubeH3));
+    return cube && H > 1 && ((dim == 2 && H <= kCubeH2) || (dim == 3 && H <= kCubeH3));
+}
+
+// Whether it is the faster one.  With the powers 1 to 5 it always is.  A
+// general power is bound by pow itself, and the staged kernel's strips of 32
+// columns evaluate it for the places beyond a narrow grid too: there it gains by
+// the half of the offsets it leaves out on a torus, and on the smallest calls,
+// which it spreads over more warps.  us, thread per cell / staged, p = 2.5: Neumann
+// 64^2 H = 8 155 / 93, 16 x 64^2 535 / 646, 16 x 256^2 7490 / 7810, 3-D 16 x 16^3 H = 4 1010 /
+// 2310; periodic 16 x 256^2 7580 / 3970, 16^3 228 / 150, 16 x 16^3 1030 / 1180, 16 x (24 x 40 x
+// 20) 4350 / 3050.
+bool staged_pays(const StructGeom& G, int dim, int bc, double p, int members) {
+    if (p == 1.0 || p == 2.0 || p == 3.0 || p == 4.0 || p == 5.0) {
+        return true;
+    }
+    const int width = (G.n[0] + 31) / 32 * 32;
+    const bool small = (long long)width * G.n[1] * G.n[2] * members <= 8192;
+    return bc == ALS_BC_PERIODIC ? small || 2 * G.n[0] > width : small && dim == 2;
 }
 
 template<class T, int DIM, int BC, int P, bool CUBE>
@@ -400,7 +433,7 @@ cudaError_t launch(const T* states, long long stride, const StructGeom& G, int n
     const int tiles = G.tiles[0] * G.tiles[1] * G.tiles[2];
     dim3 grid(tiles, nvar, members);
     if constexpr (CUBE && DIM > 1) {
-        if (staged_cube(DIM, CUBE, H)) {
+        if (G.staged) {
             constexpr int HM = DIM == 2 ? kCubeH2 : kCubeH3;
             const int r = 2 * (H - 1);
             const size_t smem = sizeof(double) * size_t(G.tile[0] + r) * (G.tile[1] + r) *
@@ -408,10 +441,12 @@ cudaError_t launch(const T* states, long long stride, const StructGeom& G, int n
             const bool share = G.tile[1] / 4 * G.tile[2] < kWarps;
             auto kernel = share ? structure_cube_kernel<T, DIM, BC, P, HM, true>
                                 : structure_cube_kernel<T, DIM, BC, P, HM, false>;
-            const cudaError_t err = cudaFuncSetAttribute(kernel,
-                cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (err != cudaSuccess) {
-                return err;
+            if (smem + 1024 > 48 * 1024) {   // beyond the default, the static part included
+                const cudaError_t err = cudaFuncSetAttribute(kernel,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+                if (err != cudaSuccess) {
+                    return err;
+                }
             }
             kernel<<<grid, kThreads, smem, s>>>(states, stride, G, nvar, H, p, partial);
             return cudaGetLastError();
@@ -496,20 +531,21 @@ extern "C" int als_structure_functions(const als_grid* grid, int boundary, int k
     const int shapes[3][3] = {{256, 1, 1}, {16, 16, 1}, {8, 8, 4}};
     const int staged[3][3] = {{0, 0, 0}, {CubeTile<2>::X, CubeTile<2>::Y, CubeTile<2>::Z},
         {CubeTile<3>::X, CubeTile<3>::Y, CubeTile<3>::Z}};
-    const bool cube = kind == ALS_STRUCTURE_CUBE;
+    G.staged = staged_cube(dim, kind == ALS_STRUCTURE_CUBE, H) &&
+        staged_pays(G, dim, boundary, p, members);
     for (int d = 0; d < 3; ++d) {
-        G.tile[d] = (staged_cube(dim, cube, H) ? staged : shapes)[dim - 1][d];
+        G.tile[d] = (G.staged ? staged : shapes)[dim - 1][d];
         G.tiles[d] = (G.n[d] + G.tile[d] - 1) / G.tile[d];
     }
-    if (staged_cube(dim, cube, H)) {
+    if (G.staged) {
         // halve the tile along y, then z, while that trims the padded cells by
-        // an eighth or the blocks do not make two per SM
+        // an eighth or the blocks do not make one per SM
         auto padded = [&](int d, int t) { return (long long)(G.n[d] + t - 1) / t * t; };
         auto blocks = [&]() { return (long long)G.tiles[0] * G.tiles[1] * G.tiles[2] * nvar * members; };
         for (int d = 1; d < dim; ++d) {
             const int least = d == 1 ? 4 : 1;
             while (G.tile[d] > least && (8 * padded(d, G.tile[d]) > 9 * padded(d, G.tile[d] / 2) ||
-                                            blocks() < 2 * 148)) {
+                                            blocks() < 148)) {
                 G.tile[d] /= 2;
                 G.tiles[d] = (G.n[d] + G.tile[d] - 1) / G.tile[d];
             }

@@ -29,3 +29,18 @@ def test_structure_cube_tile_edges(c_oracle, dim, n, members, bc, H):
     for m in (0, members - 1):
         ref = c_oracle.structure_cube(dim, n, 2, bc, H, 1.0, st[m])
         np.testing.assert_allclose(out[m], ref, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("dim,n,members", [(2, (16, 16), 1), (2, (40, 37), 30), (2, (70, 64), 2), (3, (16, 9, 8), 1),
+                                           (3, (20, 18, 17), 6)])
+@pytest.mark.parametrize("bc", ["periodic", "neumann"])
+@pytest.mark.parametrize("H,p", [(4, 2.5), (5, 0.5)])
+def test_structure_cube_general_powers(c_oracle, dim, n, members, bc, H, p):
+    """Powers that call pow, on both sides of the rule between the staged
+    kernel and a thread per cell (pow is within 2 units in the last place of
+    either library: 1e-12 as above)."""
+    st = _states(dim, n, 2, members, 17 * dim + H)
+    out = structure_functions(torch.from_numpy(st).cuda(), dim, n, 2, bc, "cube", H, p).cpu().numpy()
+    for m in (0, members - 1):
+        ref = c_oracle.structure_cube(dim, n, 2, bc, H, p, st[m])
+        np.testing.assert_allclose(out[m], ref, rtol=1e-12, atol=0)
