@@ -239,16 +239,23 @@ inline cudaError_t launch_stage_unit(const StageLauncher (&units)[kReconGroups],
 template<class R, int RECON, int FLUX, bool RK3>
 cudaError_t launch_line_one(const LineParams& P, int members, int blocks, cudaStream_t stream,
     int* clusters) {
-    auto kernel = line_kernel<R, RECON, FLUX, RK3>;
     const size_t smem = LineLayout<R, RECON, FLUX>::smem(P.stride);
+    // a thread per face of the largest piece, up to the block's limit: the wide
+    // block where it takes fewer passes (each a third longer), or shares SMs
+    const int faces = P.stride - 2 * P.ghosts + 1;
+    auto passes = [&](int threads) { return (faces + threads - 1) / threads; };
+    const bool wide = faces > kLineThreads
+        ? 13 * passes(kLineThreadsWide) < 10 * passes(kLineThreads)
+        : (long long)members * blocks > 148;
+    const int most = wide ? kLineThreadsWide : kLineThreads;
+    const int threads = std::min((faces + 31) / 32 * 32, most);
+    auto kernel = wide ? line_kernel<R, RECON, FLUX, RK3, kLineThreadsWide>
+                       : line_kernel<R, RECON, FLUX, RK3, kLineThreads>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
         int(smem));
     if (err != cudaSuccess) {
         return err;
     }
-    // a thread per face of the largest piece, up to kLineThreads
-    const int faces = P.stride - 2 * P.ghosts + 1;
-    const int threads = faces < kLineThreads ? (faces + 31) / 32 * 32 : kLineThreads;
     cudaLaunchAttribute cluster;
     cluster.id = cudaLaunchAttributeClusterDimension;
     cluster.val.clusterDim.x = unsigned(blocks);

@@ -38,7 +38,14 @@ struct LineParams {
     double gamma;
 };
 
-constexpr int kLineThreads = 288;     // most threads of a block: the 257 faces of 256 cells in one pass
+// Most threads of a block.  The kernel is built for two numbers: 256 threads may
+// have 255 registers each (FP64 uses 194), 288, the 257 faces of 256 cells in one
+// pass, share a quarter of the SM's registers three warps at a time (168 each,
+// which also lets more blocks share an SM).  FP64 WENO2, us per RK3 step, 256 / 288: 1
+// line of 1024 cells in pieces of 128 7.3 / 7.4, of 256 9.2 / 8.4, 148 lines in pieces
+// of 512 12.5 / 11.7, of 1024 18.5 / 19.8; 4096 lines of 128 cells 190 / 108.
+constexpr int kLineThreads = 256;
+constexpr int kLineThreadsWide = 288;
 constexpr int kLineBlocks = 8;        // blocks per cluster, at most (the portable size)
 constexpr int kLineCells = 1024;      // cells of a block's piece, at most
 
@@ -61,8 +68,8 @@ __device__ __forceinline__ unsigned long long warp_max_bits(double w) {
     return ((unsigned long long)top << 32) | lo;
 }
 
-template<class R, int RECON, int FLUX, bool RK3>
-__global__ void __launch_bounds__(kLineThreads, 1) line_kernel(const LineParams P) {
+template<class R, int RECON, int FLUX, bool RK3, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) line_kernel(const LineParams P) {
     namespace cg = cooperative_groups;
     typedef LineLayout<R, RECON, FLUX> Lay;
     constexpr int NV = Lay::NV;
