@@ -305,9 +305,12 @@ __global__ void __launch_bounds__(256) region_sums(const R* states, long long pl
 //   n = n_prev + k, d = mean_k - mean, mean += d*k/n, m2 += m2_k + d*d*n_prev*k/n.
 // K > 0: exactly K members, whose values a thread keeps in registers between
 // the two passes, so that each state is read once and all its loads are in
-// flight together (the two sums add in the same order either way).
-// 256 FP32 states of 4 x 260^2 into a new accumulator: 1.38 -> 0.16 ms (with the
-// pooled accumulator of als_stats_create).
+// flight together (the two sums add in the same order either way).  us per
+// addition of 64 states, two passes (the second from L2) / registers: FP64 1e6
+// elements 149 / 123, 4.2e6 570 / 454; FP32 4e3 elements 17 / 15, 270,400 27 / 28, 1e6 78
+// / 106: the FP32 values are cheap to read twice, and the registers cost the warps
+// that hide it.  256 FP32 states of 4 x 260^2 into a new accumulator: 1.38 -> 0.15 ms (its
+// arrays kept from the one before, see array_alloc).
 template<class R, int K>
 __global__ void __launch_bounds__(256) welford_merge(const R* states, long long count,
     int members, long long member_stride, double* mean, double* m2, long long n_prev) {

@@ -2,6 +2,7 @@
 // mirror one virtual call of the reference interfaces each, the fused
 // solver that runs whole time steps of one grid or of several grid levels
 // on the device, and the FP64 ensemble statistics.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -391,15 +392,110 @@ cudaError_t scratch_free(void* ptr, cudaStream_t stream) {
     return cudaFreeAsync(ptr, stream);
 }
 
-void scratch_bound() {
-    cudaMemPool_t pool = nullptr;
-    unsigned long long reserved = 0;
-    if (scratch_pool(&pool) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
-        reserved > kScratchKeep) {
-        cudaMemPoolTrimTo(pool, kScratchKeep);
+} // namespace als
+
+namespace {
+
+// Accumulator arrays that ended unseen, kept for the next accumulator of their
+// size: a cudaMalloc and cudaFree per accumulator cost more than adding a few hundred
+// states.  They are cudaMalloc's, so an accumulator's pointers (als_stats_moments) work with
+// peer access and cudaIpcGetMemHandle as any others; arrays whose pointers were handed out
+// are freed and not kept.  At most kKeptBytes per device, in arrays of up to kKeptArray;
+// als_scratch_trim and a failed allocation give them back.  A kept array is recognised by
+// its buffer id, which no other allocation ever has: one that a device reset took away is
+// forgotten.
+constexpr size_t kKeptBytes = size_t(256) << 20;
+constexpr size_t kKeptArray = size_t(64) << 20;
+struct KeptArray {
+    int device;
+    void* ptr;
+    size_t bytes;
+    unsigned long long id;
+};
+std::mutex g_kept_mutex;
+std::vector<KeptArray> g_kept;
+
+// The id of the allocation at `ptr`, 0 when there is none.
+unsigned long long buffer_id(const void* ptr) {
+    typedef CUresult (*GetAttribute)(void*, CUpointer_attribute, CUdeviceptr);
+    static GetAttribute get = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        return cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault,
+                   &found) == cudaSuccess && found == cudaDriverEntryPointSuccess
+            ? reinterpret_cast<GetAttribute>(fn) : nullptr;
+    }();
+    unsigned long long id = 0;
+    return get && get(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, reinterpret_cast<CUdeviceptr>(ptr)) ==
+            CUDA_SUCCESS ? id : 0;
+}
+
+// Frees the current device's kept arrays down to `keep` bytes.
+void free_kept(int device, size_t keep) {
+    std::lock_guard<std::mutex> lock(g_kept_mutex);
+    size_t total = 0;
+    for (const KeptArray& k : g_kept) {
+        total += k.device == device ? k.bytes : 0;
+    }
+    for (size_t i = 0; i < g_kept.size() && total > keep;) {
+        if (g_kept[i].device != device) {
+            ++i;
+            continue;
+        }
+        if (buffer_id(g_kept[i].ptr) == g_kept[i].id) {
+            cudaFree(g_kept[i].ptr);
+        }
+        total -= g_kept[i].bytes;
+        g_kept.erase(g_kept.begin() + i);
     }
 }
+
+// `bytes` on the current device, kept or new.
+cudaError_t array_alloc(double** ptr, int device, size_t bytes) {
+    {
+        std::lock_guard<std::mutex> lock(g_kept_mutex);
+        for (size_t i = 0; i < g_kept.size();) {
+            if (g_kept[i].device != device || g_kept[i].bytes != bytes) {
+                ++i;
+                continue;
+            }
+            const KeptArray k = g_kept[i];
+            g_kept.erase(g_kept.begin() + i);
+            if (buffer_id(k.ptr) == k.id) {
+                *ptr = static_cast<double*>(k.ptr);
+                return cudaSuccess;
+            }
+        }
+    }
+    cudaError_t err = cudaMalloc((void**)ptr, bytes);
+    if (err == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        free_kept(device, 0);
+        err = cudaMalloc((void**)ptr, bytes);
+    }
+    return err;
+}
+
+// Keeps or frees an array of the current device that no work uses any more.
+void array_free(void* ptr, int device, size_t bytes, bool seen) {
+    const unsigned long long id = seen || bytes > kKeptArray ? 0 : buffer_id(ptr);
+    if (id) {
+        std::lock_guard<std::mutex> lock(g_kept_mutex);
+        size_t total = bytes;
+        for (const KeptArray& k : g_kept) {
+            total += k.device == device ? k.bytes : 0;
+        }
+        if (total <= kKeptBytes) {
+            g_kept.push_back(KeptArray{device, ptr, bytes, id});
+            return;
+        }
+    }
+    cudaFree(ptr);
+}
+
+} // namespace
+
+namespace als {
 } // namespace als
 
 extern "C" {
@@ -417,10 +513,21 @@ int als_scratch_trim(int device, unsigned long long keep_bytes) {
         std::lock_guard<std::mutex> lock(als::g_scratch_mutex);
         pool = als::g_scratch_pools[device];
     }
-    if (!pool) {
+    bool kept = false;
+    {
+        std::lock_guard<std::mutex> lock(g_kept_mutex);
+        for (const KeptArray& k : g_kept) {
+            kept = kept || k.device == device;
+        }
+    }
+    if (!pool && !kept) {
         return ALS_OK;
     }
     DeviceGuard guard(device);
+    free_kept(device, size_t(keep_bytes));
+    if (!pool) {
+        return ALS_OK;
+    }
     ALS_CUDA(cudaMemPoolTrimTo(pool, size_t(keep_bytes)));
     return ALS_OK;
 }
@@ -2068,24 +2175,22 @@ struct als_stats {
     int device = 0;
     long long count = 0;          // elements per state
     long long n = 0;              // states accumulated
-    double* mean = nullptr;       // one allocation for both arrays
+    double* mean = nullptr;
     double* m2 = nullptr;
-    bool pooled = false;
+    bool seen = false;            // the arrays' pointers were handed out
     ~als_stats() {
-        if (!mean) {
+        if (!mean && !m2) {
             return;
         }
         int prev = 0;
         cudaGetDevice(&prev);
         cudaSetDevice(device);
-        if (pooled) {
-            // work on any stream may still use the arrays (cudaFree, which the
-            // larger ones take, waits for it too)
-            cudaDeviceSynchronize();
-            als::scratch_free(mean, nullptr);
-            als::scratch_bound();
-        } else {
-            cudaFree(mean);
+        // work on any stream may still use the arrays (cudaFree waits for it too)
+        cudaDeviceSynchronize();
+        for (double* p : {mean, m2}) {
+            if (p) {
+                array_free(p, device, sizeof(double) * size_t(count), seen);
+            }
         }
         cudaSetDevice(prev);
     }
@@ -2096,13 +2201,16 @@ namespace {
 template<class R>
 int stats_merge_states(als_stats* st, const R* states, int members, long long member_stride,
     cudaStream_t s) {
-    // chunks of at most 64 states: a whole one stays in registers between
-    // its two passes, the last one in L2
+    // chunks of at most 64 states; a whole one of FP64, or of FP32 whose elements
+    // have a thread each at once, stays in registers between its two passes (more FP32
+    // elements are faster in two: see welford_merge)
     for (int first = 0; first < members; first += 64) {
         const int k = std::min(64, members - first);
-        auto merge = k == 64 ? als::welford_merge<R, 64> : als::welford_merge<R, 0>;
-        const long long blocks = std::min<long long>((st->count + 255) / 256, 1LL << 20);
-        merge<<<int(blocks), 256, 0, s>>>(states + (long long)first * member_stride, st->count, k,
+        const bool whole = k == 64 && (sizeof(R) == 8 || st->count <= 148LL * 512);
+        auto merge = whole ? als::welford_merge<R, 64> : als::welford_merge<R, 0>;
+        const int blocks = whole ? int(std::min<long long>((st->count + 255) / 256, 1LL << 20))
+                                 : grid_blocks(st->count, 256);
+        merge<<<blocks, 256, 0, s>>>(states + (long long)first * member_stride, st->count, k,
             member_stride, st->mean, st->m2, st->n);
         ALS_CUDA(cudaGetLastError());
         st->n += k;
@@ -2126,17 +2234,11 @@ int als_stats_create(long long count, int device, als_stats** out) {
     st->device = device;
     st->count = count;
     DeviceGuard guard(device);
-    // accumulators up to 64 MiB come from the library's pool: a cudaMalloc and
-    // cudaFree per accumulator cost more than adding a few hundred states
-    const size_t bytes = 2 * sizeof(double) * size_t(count);
-    st->pooled = bytes <= (64u << 20);
-    if (st->pooled) {
-        ALS_CUDA(als::scratch_alloc((void**)&st->mean, bytes, nullptr));
-    } else {
-        ALS_CUDA(cudaMalloc((void**)&st->mean, bytes));
-    }
-    st->m2 = st->mean + count;
+    const size_t bytes = sizeof(double) * size_t(count);
+    ALS_CUDA(array_alloc(&st->mean, device, bytes));
+    ALS_CUDA(array_alloc(&st->m2, device, bytes));
     ALS_CUDA(cudaMemsetAsync(st->mean, 0, bytes, nullptr));
+    ALS_CUDA(cudaMemsetAsync(st->m2, 0, bytes, nullptr));
     // the first addition may come on any stream
     ALS_CUDA(cudaStreamSynchronize(nullptr));
     *out = st.release();
@@ -2214,6 +2316,7 @@ int als_stats_moments(als_stats* st, long long* n, double** mean, double** m2) {
     if (n) {
         *n = st->n;
     }
+    st->seen = st->seen || mean || m2;
     if (mean) {
         *mean = st->mean;
     }

@@ -20,8 +20,4 @@ cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t stream);
 // Returns memory from scratch_alloc to the library's pool, ordered on `stream`.
 cudaError_t scratch_free(void* ptr, cudaStream_t stream);
 
-// Gives the current device's unused pool memory beyond kScratchKeep back.
-constexpr size_t kScratchKeep = size_t(1) << 30;
-void scratch_bound();
-
 } // namespace als

@@ -64,7 +64,8 @@ int als_version(void);
  * (functionals, structure functions, region sums) comes from one retaining
  * pool per device: it keeps the largest amount any call needed until the
  * process exits, hidden from other allocators.  This hands the unused part
- * of `device`'s pool back until at most `keep_bytes` stay reserved.  It has
+ * of `device`'s pool back until at most `keep_bytes` stay reserved, and the
+ * arrays kept of ended accumulators (als_stats, at most 256 MiB) likewise.  It has
  * no counterpart in the reference (its volumes allocate per object). */
 int als_scratch_trim(int device, unsigned long long keep_bytes);
 
@@ -322,7 +323,9 @@ int als_stats_add_solver(als_stats* st, als_solver* s, int level);
 /* Chan merge of another accumulator's (n, mean, M2) (device arrays), e.g.
  * from another GPU. */
 int als_stats_merge(als_stats* st, long long n, const double* mean, const double* m2, void* stream);
-/* n and device pointers of the running mean and M2. */
+/* n and device pointers of the running mean and M2: two cudaMalloc
+ * allocations, open to peer access and cudaIpcGetMemHandle, until
+ * als_stats_destroy. */
 int als_stats_moments(als_stats* st, long long* n, double** mean, double** m2);
 /* Writes mean and variance (device arrays of `count` doubles; either may be NULL). */
 int als_stats_result(als_stats* st, double* mean, double* variance, void* stream);
