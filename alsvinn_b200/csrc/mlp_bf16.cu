@@ -156,7 +156,7 @@ int launch_gemm(const GemmArgs& a, int n_valid, cudaStream_t s, int splits = 1,
     if (a.M % kTileM || a.N % BN || a.K % kChunkK || a.K <= 0 || splits < 1 || splits > 65535) {
         return mlp_fail(ALS_E_INVALID, "GEMM shape is not a multiple of the tile");
     }
-    constexpr int smem = gemm_smem_bytes<BN>();   // limit set by configure_kernels()
+    const int smem = gemm_smem_bytes<BN>(a.K / kChunkK);   // limit set by configure_kernels()
     dim3 grid(a.M / kTileM, a.N / BN, splits);
     cudaLaunchAttribute overlap;
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
