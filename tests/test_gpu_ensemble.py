@@ -86,8 +86,9 @@ def test_level_order_and_tuning_do_not_change_results():
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("integ", ["rungekutta3", "rungekutta2", "forwardeuler"])
 def test_tile_shape_per_level_does_not_change_results(precision, integ):
-    """Levels on the 16x16 tile, the 32x16 tile or a mix (one launch per
-    shape and stage), and persistent launches over them, give the same bits."""
+    """Levels on the 16x16 tile, the kernel that their size takes (a thread per
+    face) or a mix (one launch per kernel and stage), and persistent launches
+    over them, give the same bits."""
     g = ghost_cells("weno2")
     states = _level_states(LEVELS, g, 800)
     base, base_info = _run_levels(LEVELS, states, precision=precision, integrator=integ)
@@ -205,19 +206,22 @@ def test_uq_oracle_members_equal_single_runs_at_full_size(sample):
     assert y[0] == z["y"][sample]
 
 
-Z_CASES = [((20, 18, 40), "weno2", "hll3", "rungekutta3", "periodic", 2),
-           ((17, 16, 33), "eno2", "hll", "rungekutta2", "neumann", 1),
-           ((16, 21, 18), "mc", "central", "forwardeuler", "periodic", 3),
-           ((18, 17, 35), "wenof2", "hll3", "rungekutta3", "neumann", 1),
-           ((16, 16, 16), "none", "hll", "rungekutta3", "periodic", 2),
-           ((19, 16, 20), "mm", "hll3", "rungekutta2", "periodic", 1)]
+# above 100,000 cells in all, where shape 1 marches; ragged against the 16 x 15
+# columns and the segments
+Z_CASES = [((41, 37, 34), "weno2", "hll3", "rungekutta3", "periodic", 2),
+           ((33, 31, 100), "eno2", "hll", "rungekutta2", "neumann", 1),
+           ((35, 30, 33), "mc", "central", "forwardeuler", "periodic", 3),
+           ((49, 46, 47), "wenof2", "hll3", "rungekutta3", "neumann", 1),
+           ((32, 46, 35), "none", "hll", "rungekutta3", "periodic", 2),
+           ((61, 48, 36), "mm", "hll3", "rungekutta2", "periodic", 1),
+           ((50, 45, 47), "mm", "hll", "rungekutta3", "neumann", 1)]
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("n,recon,flux,integ,bc,members", Z_CASES,
                          ids=["%s-%s-%s-%s" % (c[1], c[2], c[3], c[4]) for c in Z_CASES])
 def test_z_marching_3d_tiles_equal_the_box_tiles(n, recon, flux, integ, bc, members, precision):
-    """3-D shape 1 (16x16 columns marching along z in segments) gives the
+    """3-D shape 1 (16x15 columns marching along z in segments) gives the
     bits of shape 0 (8x8x4 boxes): every member, ghosts included, with
     partial columns and segments, both boundaries, every integrator."""
     g = ghost_cells(recon)
@@ -228,6 +232,7 @@ def test_z_marching_3d_tiles_equal_the_box_tiles(n, recon, flux, integ, bc, memb
                            integrator=integ, boundary=bc, cfl=0.4, end_time=0.02,
                            precision=precision, members=members) as sim:
             sim.set_tiles([shape])
+            assert sim.kernels() == [("tiles", "columns")[shape]]
             sim.set_state(states)
             sim.run()
             out[shape] = (sim.get_state(), [sim.info(m) for m in range(members)])
@@ -239,8 +244,8 @@ def test_z_marching_3d_tiles_equal_the_box_tiles(n, recon, flux, integ, bc, memb
 
 def test_z_marching_3d_against_the_oracle(c_oracle):
     """Shape 1 on KH-like 3-D data against the C oracle directly (WENO2 +
-    HLL3, RK3, periodic), a grid of two z segments plus a partial one."""
-    n, g = (17, 16, 70), 2
+    HLL3, RK3, periodic), a grid with partial columns and uneven segments."""
+    n, g = (35, 46, 70), 2
     st = smooth_random_state(41, 3, n, g)
     cfg = c_oracle.config(3, n, (0, 0, 0), (1, 1, 1), "hll3", "weno2", "rungekutta3", "periodic",
                           1.4)
@@ -249,7 +254,7 @@ def test_z_marching_3d_against_the_oracle(c_oracle):
                        integrator="rungekutta3", boundary="periodic", cfl=0.4, end_time=10.0,
                        max_steps=3) as sim:
         sim.set_tiles([1])
-        assert sim.tiles()["extents"][0][:2] == (16, 16)
+        assert sim.tiles()["extents"][0][:2] == (16, 16) and sim.kernels() == ["columns"]
         sim.set_state(st)
         sim.run()
         info = sim.info()

@@ -110,3 +110,43 @@ def test_adiabatic_exponents(c_oracle, gamma):
     got_ws = als.NumericalFlux(2, n, "hll3", "weno2", gamma=gamma).computeFlux(dev, out)
     np.testing.assert_array_equal(out.cpu().numpy()[:, :, g:-g, g:-g], expect[:, :, g:-g, g:-g])
     np.testing.assert_array_equal(got_ws[:2], ws[:2])
+
+
+@pytest.mark.parametrize("dim,n", [(2, (301, 263)), (2, (801, 503)), (3, (40, 36, 35)), (3, (50, 47, 44)), (1, (80000,))],
+                         ids=["small tiles", "rows", "boxes", "columns", "1-D tiles"])
+@pytest.mark.parametrize("flux", ["hll", "hll3"])
+@pytest.mark.parametrize("kind", KINDS)
+def test_every_kernel_falls_back(c_oracle, dim, n, flux, kind):
+    """The same states through the kernels of larger grids (their sizes above)."""
+    g = 2
+    rng = np.random.default_rng(KINDS.index(kind) + dim)
+    st = _states(kind, dim, rng, padded_shape(dim, n, g))
+    cfg = c_oracle.config(dim, n, [0.0] * dim, [1.0] * dim, flux, "weno2", "rungekutta3", "periodic",
+                          GAMMA)
+    with np.errstate(all="ignore"):
+        st = c_oracle.fill_ghosts(cfg, st)
+        expect, ws = c_oracle.net_flux(cfg, st)
+    dev = torch.from_numpy(st).cuda()
+    out = torch.zeros_like(dev)
+    got_ws = als.NumericalFlux(dim, n, flux, "weno2", gamma=GAMMA).computeFlux(dev, out)
+    inner = (slice(None),) + tuple(slice(g, -g) if d < dim else slice(None) for d in (2, 1, 0))
+    np.testing.assert_array_equal(out.cpu().numpy()[inner], expect[inner])
+    np.testing.assert_array_equal(got_ws[:dim], ws[:dim])
+
+
+@pytest.mark.parametrize("flux", ["hll", "hll3"])
+@pytest.mark.parametrize("kind", ["ordinary", "supersonic", "signed_zero", "tiny_momentum", "mantissas"])
+def test_line_steps_fall_back(c_oracle, flux, kind):
+    """Whole steps of a line in one launch."""
+    n = 900
+    st = _states(kind, 1, np.random.default_rng(9), padded_shape(1, (n,), 2))
+    cfg = c_oracle.config(1, (n,), [0.0], [1.0], flux, "weno2", "rungekutta3", "periodic", GAMMA)
+    with np.errstate(all="ignore"):
+        rc, expect, dts, steps, t = c_oracle.simulate(cfg, c_oracle.fill_ghosts(cfg, st), 0.4, 1e300,
+                                                      max_steps=1)
+    with als.Simulator(1, (n,), flux=flux, reconstruction="weno2", cfl=0.4, end_time=1e300, max_steps=1) as sim:
+        assert sim.kernels() == ["lines"]
+        sim.set_state(st)
+        sim.advance(1)
+        np.testing.assert_array_equal(sim.get_state()[0], expect)
+        assert sim.info()["t"] == t

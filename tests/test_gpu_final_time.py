@@ -251,8 +251,8 @@ def test_neumann_riemann_to_final_time_matches_reference(name):
 @pytest.mark.parametrize("shape", [1, 0], ids=["z-marching columns", "8x8x4 boxes"])
 def test_kh3d_to_final_time_matches_reference(shape):
     """3-D KH 48^3 to T = 2 one step at a time with each 3-D tile shape:
-    every dt and the final interior equal to the reference build's (48
-    cells along z are two z-marching segments, 32 + 16)."""
+    every dt and the final interior equal to the reference build's (110,592
+    cells: shape 1 marches)."""
     z = ft.load("kh3d48")
     n = z["n"]
     U0 = init.kelvin_helmholtz(n, z["params"], ft.GHOSTS, ft.GAMMA, dimension=3)
@@ -261,7 +261,7 @@ def test_kh3d_to_final_time_matches_reference(shape):
                        reconstruction=z["recon"], integrator=z["integrator"], boundary=z["bc"],
                        gamma=z["gamma"], cfl=z["cfl"], end_time=z["end_time"]) as sim:
         sim.set_tiles([shape])
-        assert sim.tiles()["shapes"] == [shape]
+        assert sim.tiles()["shapes"] == [shape] and sim.kernels() == [("tiles", "columns")[shape]]
         sim.set_state(U0)
         dts = _step_by_step(sim)
         info = sim.info()

@@ -1,11 +1,5 @@
-"""The stage kernels and the rules that choose between them, against the C
-oracle bit for bit, at the sizes where they can go wrong.
-
-2-D grids above 400,000 cells (FP64) march warps along y (runs of rows, strips
-of 32 columns), those below 72,000 and 3-D grids below 60,000 take a thread per
-face, 2-D grids between take 16 x 16 tiles, larger 3-D grids march blocks along z
-(segments of planes, 16 x 15 columns), 1-D RK2 / RK3 runs whole steps in a
-cluster per line.
+"""The stage kernels against the C oracle bit for bit, at the sizes where they can
+go wrong.  Which kernel runs where: test_gpu_kernel_choice.py.
 """
 import numpy as np
 import pytest
@@ -15,6 +9,7 @@ from oracle_lib import ghost_cells, smooth_random_state
 torch = pytest.importorskip("torch")
 
 import alsvinn_b200 as als  # noqa: E402
+from alsvinn_b200 import domain  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -106,6 +101,41 @@ def test_marching_steps(c_oracle, dim, n, integ, bc):
         info = sim.info()
         np.testing.assert_array_equal(sim.get_state()[0], expect)
     assert info["steps"] == steps and info["t"] == t
+
+
+MARCHING = [(2, (703, 632), (1, 4), "rows"), (2, (300, 280), (2, 1), "small tiles"),
+            (3, (60, 48, 50), (1, 2, 2), "columns"), (3, (40, 36, 35), (2, 1, 1), "tiles")]
+
+
+@pytest.mark.parametrize("dim,n,procs,kernel", MARCHING, ids=["%s-%s" % (c[3], "x".join(map(str, c[1]))) for c in MARCHING])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("bc", ["periodic", "neumann"])
+def test_persistent_and_split_launches(dim, n, procs, kernel, precision, bc):
+    """Persistent launches and a grid split into subdomains (ghost layers
+    written across them by the stage kernels) give the bits of the plain run."""
+    g = ghost_cells("weno2")
+    st = smooth_random_state(11 + dim, dim, n, g)
+    common = dict(flux="hll3", reconstruction="weno2", integrator="rungekutta3", boundary=bc, cfl=0.4,
+                  end_time=1.0, max_steps=3, precision=precision)
+    out = []
+    for blocks in (0, 1):
+        with als.Simulator(dim, n, **common) as sim:
+            assert sim.kernels() == [kernel]
+            sim.set_schedule(blocks)
+            sim.set_state(st)
+            sim.run()
+            out.append(sim.get_state()[0])
+    np.testing.assert_array_equal(out[1], out[0])
+    split = domain.SplitSimulation(dim, n, procs, **common)
+    try:
+        assert split.sim.kernels() == [kernel]
+        split.set_state(st)
+        split.run()
+        blocks = split.sim.get_state()
+        for r, dec in enumerate(split.decs):
+            np.testing.assert_array_equal(blocks[r], out[0][dec.local_slice(g)])
+    finally:
+        split.close()
 
 
 LINES = [4, 9, 63, 64, 127, 128, 129, 255, 256, 511, 513, 1000, 2047, 4097, 8192, 8193]
