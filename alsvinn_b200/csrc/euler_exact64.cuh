@@ -8,9 +8,9 @@
 // that are not zero) reports it, and the caller evaluates the plain form.
 //
 // Why the tests suffice.  With both densities and pressures in
-// [2^-60, 2^60): (gamma-1)(E - m.m/(2 rho)) = p bounds |m| by 2^90, E by
-// 2^114, velocities and speeds by 2^88; normal momenta are 0 or at least
-// 2^-700, so velocities, their Roe sums (a sum of doubles is 0 or at least
+// [2^-60, 2^60) and gamma - 1 at least 2^-20: (gamma-1)(E - m.m/(2 rho)) = p,
+// a difference rounded in the 53rd place, bounds E by 2^133, |m| and velocities
+// by 2^97 and speeds by 2^98; normal momenta are 0 or at least 2^-700, so velocities, their Roe sums (a sum of doubles is 0 or at least
 // the last place of its smallest operand) and every denominator below stay
 // far from over- and underflow.  The kinetic energy m.m/(2 rho) may be
 // subnormal, but only where it is lost against E whatever its last bits.

@@ -53,15 +53,18 @@ cudaError_t resident_blocks(int threads, size_t smem, int* blocks) {
 // there are work items.
 //
 // The solver's stages may be chained: a stage's blocks take their places while
-// the one before it ends, which hides its launch (2 to 7 %).  Not with fewer
-// blocks than the GPU holds at once: the early ones then double up on the SMs
-// that the running stage leaves free, and the stage takes as long as those
-// (TeCNO6, 256^2, 128 tiles, us per RK3 step: 119 apart, 190 chained; KH 32^2 by
-// faces 17.9 and 20.2).  `small` kernels are chained all the same: bound by
-// latency, sharing an SM costs them nothing (FP32 faces, 64^2: 18.2 and 17.5).
+// the one before it ends, which hides its launch (2 to 7 %).  With too few blocks for
+// the GPU that costs more than it gives: the early ones double up on the SMs that the
+// running stage leaves free, and the stage takes as long as those.  So a launch is chained
+// from `quarters` quarters of the blocks that the GPU holds at once.  us per RK3 step,
+// apart / chained: TeCNO6 256^2, 128 tiles, 119 / 190; FP64 faces 32^2 17.9 / 20.2, 160^2
+// (230 boxes of 296) 23 / 22; 24^3 29 / 33 (144 of 148); FP32 16 x 16 tiles 320^2 (400 of
+// 592) 27 / 30, 64 x 648 x 3 (492) 36 / 33.  Always chained: FP64 16 x 16 tiles (320^2 43 /
+// 41) and the FP32 1-D and 2-D faces, which are bound by latency, so that sharing an SM
+// costs them nothing (64^2: 18.2 / 17.5).
 template<void (*KERNEL)(StageParams)>
 cudaError_t launch_stage_blocks(int threads, size_t smem, const StageParams& P, int blocks_per_sm,
-    cudaStream_t stream, bool small = false) {
+    cudaStream_t stream, int quarters) {
     // raising the dynamic shared-memory limit is idempotent and cheap; it is
     // done on every launch so that every device the process uses is covered
     cudaError_t err = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -73,7 +76,7 @@ cudaError_t launch_stage_blocks(int threads, size_t smem, const StageParams& P, 
         return cudaSuccess;
     }
     int resident = 0;
-    if (P.counter || (P.chained && !small)) {
+    if (P.counter || (P.chained && quarters > 0)) {
         err = resident_blocks<KERNEL>(threads, smem, &resident);
         if (err != cudaSuccess) {
             return err;
@@ -101,7 +104,7 @@ cudaError_t launch_stage_blocks(int threads, size_t smem, const StageParams& P, 
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     config.attrs = &chained;
-    config.numAttrs = P.chained && (small || blocks >= resident) ? 1 : 0;
+    config.numAttrs = P.chained && 4 * blocks >= (long long)quarters * resident ? 1 : 0;
     return cudaLaunchKernelEx(&config, KERNEL, P);
 }
 
@@ -114,19 +117,19 @@ cudaError_t launch_stage_one(const StageParams& P, int b, cudaStream_t s) {
     if constexpr (SHAPE == kFacesKernel) {
         typedef FaceLayout<R, DIM, RECON, FLUX> Lay;
         return launch_stage_blocks<faces_kernel<R, DIM, RECON, FLUX, KIND>>(Lay::THREADS, Lay::SMEM,
-            P, b, s, sizeof(R) == 4 && DIM < 3);
+            P, b, s, DIM == 3 ? 4 : (sizeof(R) == 4 ? 0 : 3));
     } else if constexpr (SHAPE == kPlanesKernel) {
         typedef ZLayout<R, RECON, FLUX> Lay;
         return launch_stage_blocks<zmarch_kernel<R, RECON, FLUX, KIND>>(Lay::THREADS, Lay::SMEM, P,
-            b, s);
+            b, s, 4);
     } else if constexpr (marches_rows(DIM, FLUX, SHAPE)) {
         typedef RowLayout<R, RECON, FLUX> Lay;
         // a block of the schedule stands for eight of these warps
-        return launch_stage_blocks<rows_kernel<R, RECON, FLUX, KIND>>(32, Lay::SMEM, P, 8 * b, s);
+        return launch_stage_blocks<rows_kernel<R, RECON, FLUX, KIND>>(32, Lay::SMEM, P, 8 * b, s, 3);
     } else {
         typedef StageLayout<R, DIM, RECON, FLUX, SHAPE> Lay;
         return launch_stage_blocks<stage_kernel<R, DIM, RECON, FLUX, KIND, SHAPE>>(Lay::THREADS,
-            Lay::SMEM, P, b, s);
+            Lay::SMEM, P, b, s, DIM == 3 ? 4 : (DIM == 2 && SHAPE == 1 && sizeof(R) == 8 ? 0 : 3));
     }
 }
 

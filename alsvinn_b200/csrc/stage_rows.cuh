@@ -14,9 +14,10 @@
 //      column's left face, the left state beyond the last column) is formed
 //      for all rows of the run at once, one row per lane, before the walk.
 // So the reconstructed states and fluxes stay in registers, there is no
-// block barrier.  FP64 WENO2 + HLL3, per cell and stage: 690 FP64 instructions
-// of 1,310 (the tiled kernel with plain divisions: 895 of 2,650); FP64 pipe
-// 60 % busy; FP32 per cell 730, of the issue slots 80 %.  Ms per RK3 step: KH
+// block barrier.  FP64 WENO2 + HLL3, per cell and stage: 670 to 701 FP64
+// instructions of 1,207 to 1,292 (the tiled kernel with plain divisions: 895 of
+// 2,650); FP64 pipe 55 to 58 % busy; FP32 642 to 750, 73 to 78 % of the issue
+// slots.  Ms per RK3 step: KH
 // 1024^2 FP64 0.279 (tiled) -> 0.235, 4096^2 4.66 (tiled, plain divisions) -> 2.83,
 // 512 x 256^2 FP32 members 4.35 -> 2.21.
 //
