@@ -539,13 +539,14 @@ extern "C" int als_structure_functions(const als_grid* grid, int boundary, int k
     }
     if (G.staged) {
         // halve the tile along y, then z, while that trims the padded cells by
-        // an eighth or the blocks do not make one per SM
+        // an eighth or the blocks are fewer than 256 (128^2, one state, H = 2: 256
+        // blocks 32 us, 512 42; 3-D 32^3, H = 5: 160 blocks 104 us, 320 83)
         auto padded = [&](int d, int t) { return (long long)(G.n[d] + t - 1) / t * t; };
         auto blocks = [&]() { return (long long)G.tiles[0] * G.tiles[1] * G.tiles[2] * nvar * members; };
         for (int d = 1; d < dim; ++d) {
             const int least = d == 1 ? 4 : 1;
             while (G.tile[d] > least && (8 * padded(d, G.tile[d]) > 9 * padded(d, G.tile[d] / 2) ||
-                                            blocks() < 148)) {
+                                            blocks() < 256)) {
                 G.tile[d] /= 2;
                 G.tiles[d] = (G.n[d] + G.tile[d] - 1) / G.tile[d];
             }
