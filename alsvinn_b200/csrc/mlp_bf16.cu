@@ -152,11 +152,12 @@ void launch_pack(const float* x, long long rows, int nin, __nv_bfloat16* xb, lon
 // launch may overlap its end (the kernel waits for it before it reads).
 template <int BN, int EPI>
 int launch_gemm(const GemmArgs& a, int n_valid, cudaStream_t s, int splits = 1,
-                bool chained = false) {
+                bool chained = false, bool compact = false) {
     if (a.M % kTileM || a.N % BN || a.K % kChunkK || a.K <= 0 || splits < 1 || splits > 65535) {
         return mlp_fail(ALS_E_INVALID, "GEMM shape is not a multiple of the tile");
     }
-    const int smem = gemm_smem_bytes<BN>(a.K / kChunkK);   // limit set by configure_kernels()
+    // limit set by configure_kernels()
+    const int smem = compact ? gemm_smem_bytes<BN>(a.K / kChunkK) : gemm_smem_bytes<BN>();
     dim3 grid(a.M / kTileM, a.N / BN, splits);
     cudaLaunchAttribute overlap;
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -337,7 +338,7 @@ int forward_hidden(als_mlp* s, const __nv_bfloat16* x, long long rows_pad,
                              : (launch_tma_forward<4, false>(ta, s->tm_w[l], a, hw, hb, nullptr, 0, st)));
             }
         } else if (zs || L.out % 128 != 0) {
-            MLP_TRY((launch_gemm<64, EPI_FORWARD>(a, L.out, st, 1, zs && l > 0)));
+            MLP_TRY((launch_gemm<64, EPI_FORWARD>(a, L.out, st, 1, zs && l > 0, !zs)));
         } else if (L.out % 256 != 0) {
             MLP_TRY((launch_gemm<128, EPI_FORWARD>(a, L.out, st)));
         } else {

@@ -16,10 +16,12 @@ __host__ __device__ constexpr int gemm_stages() {
     return BN == 64 ? 4 : 2;
 }
 
-// Shared memory for `chunks` chunks of K.  The 64-wide tiles take what their K
-// needs (and their epilogue's tile), so that more of them share an SM: with four
-// stages whatever the K, 1e6 rows of a 64-wide network took 570 us instead of 520.  The wide ones
-// keep two, which is also as many CTAs as their TMEM columns allow.
+// Shared memory for `chunks` chunks of K.  The 64-wide tiles of an inference take
+// what their K needs (and their epilogue's tile), so that more of them share an SM:
+// with four stages whatever the K, 1e6 rows of a 64-wide network took 570 us instead
+// of 500.  A training step's keep all four: they are few, and two of them sharing an SM
+// where others are idle cost 2 to 3 %.  The wide tiles keep two, which is also as many
+// CTAs as their TMEM columns allow.
 template <int BN>
 constexpr int gemm_smem_bytes(int chunks = gemm_stages<BN>()) {
     const int stages = BN == 64 && chunks < gemm_stages<BN>() ? chunks : gemm_stages<BN>();
