@@ -171,18 +171,18 @@ long long region_cells(const als::GridDesc& gd) {
     return (long long)(gd.hi[0] - gd.lo[0]) * (gd.hi[1] - gd.lo[1]) * (gd.hi[2] - gd.lo[2]);
 }
 
-// Boxes of the thread-per-face kernel that cover the region of a grid.
-long long face_boxes(const als::GridDesc& gd, int dim, int precision) {
-    long long boxes = 1;
+// Tiles of kernel `kernel` that cover the region of a grid.
+long long cover(const als::GridDesc& gd, int dim, int kernel, int precision) {
+    long long count = 1;
     for (int d = 0; d < dim; ++d) {
-        const int t = tile_extent(precision, dim, d, als::kFacesKernel);
-        boxes *= (gd.hi[d] - gd.lo[d] + t - 1) / t;
+        const int t = tile_extent(precision, dim, d, kernel);
+        count *= (gd.hi[d] - gd.lo[d] + t - 1) / t;
     }
-    return boxes;
+    return count;
 }
 
-// Kernel for levels of tile shape `shape` with `cells` cells in all, `boxes`
-// boxes of the thread-per-face kernel.  A thread per face has the least latency
+// Kernel for levels of tile shape `shape` with `cells` cells in all, in `boxes`
+// boxes of the thread-per-face kernel or `tiles` of shape 0's tiles.  A thread per face has the least latency
 // but repeats work at its boxes' edges, so it runs the smallest grids, up to as
 // many boxes as the GPU takes in one or two rounds; warps that march along y (2-D)
 // and columns that march along z do the least work but need long runs, so they
@@ -198,13 +198,13 @@ long long face_boxes(const als::GridDesc& gd, int dim, int precision) {
 // (152) 18.7 / 23.8, 192^2 29.4 / 29.3, 256^2 32 / 31.  TeCNO1 has 32 x 16 tiles on the
 // larger grids (1024^2, FP64: 326, marching 388).
 //   3-D (148 boxes a round), thread per face / 8 x 8 x 4 boxes / marching: FP64, WENO2
-// 24^3 (144) 33 / 45 / 67, 28^3 (280) 47 / 51 / 76, 32^3 (352) 61 / 52 / 76, 48^3 146 / 79 /
-// 81; ENO3 24^3 34 / 45, 28^3 49 / 46 (face, boxes); FP32, WENO2 24^3 27 / 31 / 47, 28^3
+// 24^3 (144) 33 / 45 / 67, 28^3 (280) 47 / 51 / 76, 32^3 (352) 61 / 52 / 76, 48^3 (432
+// tiles) 146 / 79 / 81; ENO3 24^3 34 / 45, 28^3 49 / 46 (face, boxes); FP32, WENO2 24^3 27 / 31 / 47, 28^3
 // 35 / 33 / 51, 40^3 71 / 35 / 53, 48^3 108 / 58 / 54.
 constexpr long long kTilesCells2[2] = {400000, 270000};   // FP64, FP32
-constexpr long long kBoxesCells3 = 100000;
+constexpr long long kTiles3 = 400;
 int choose_kernel(int dim, int recon, int flux, int shape, int n0, long long cells, long long boxes,
-    int precision) {
+    long long tiles, int precision) {
     if (als::stencil_flux(flux) || (dim == 2 && shape != 0)) {
         return shape;
     }
@@ -222,7 +222,7 @@ int choose_kernel(int dim, int recon, int flux, int shape, int n0, long long cel
     if (boxes <= (fp64 && als::recon_ghosts(recon) <= 2 ? 148 * 2 : 148)) {
         return als::kFacesKernel;
     }
-    return shape == 1 && cells > kBoxesCells3 ? als::kPlanesKernel : 0;
+    return shape == 1 && tiles > kTiles3 ? als::kPlanesKernel : 0;
 }
 
 // The tile shape a configuration starts on: in 3-D the columns marching along
@@ -237,7 +237,8 @@ als::GridDesc plan_region(int dim, const int* n, int g, const int* lo, const int
     int flux, int members, int* kernel) {
     als::GridDesc gd = make_grid(dim, n, g, lo, hi);
     *kernel = choose_kernel(dim, recon, flux, default_shape(dim, recon, flux), gd.hi[0] - gd.lo[0],
-        region_cells(gd) * members, face_boxes(gd, dim, ALS_FP64) * members, ALS_FP64);
+        region_cells(gd) * members, cover(gd, dim, als::kFacesKernel, ALS_FP64) * members,
+        cover(gd, dim, 0, ALS_FP64) * members, ALS_FP64);
     gd = make_grid(dim, n, g, lo, hi, ALS_FP64, *kernel);
     if (als::marches_rows(dim, flux, *kernel)) {
         split_runs(gd, run_rows(strip_rows(gd) * members, ALS_FP64));
@@ -868,6 +869,7 @@ struct als_solver {
     als::StepState* host_state = nullptr;  // pinned mirror
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph = nullptr;
+    bool capturing = false;       // the step being enqueued goes into the graph
     int graph_steps = 0;
     int graph_cur = 0;
 
@@ -961,7 +963,7 @@ als::StageParams solver_params(const als_solver* s, Pick pick, int kernel) {
     P.bc = s->cfg.boundary;
     P.write_ghosts = 1;
     P.gamma = s->cfg.gamma;
-    P.chained = 1;
+    P.chained = s->capturing ? 1 : 2;
     P.counter = s->blocks_per_sm > 0 ? s->counter : nullptr;
     finish_params(P);
     return P;
@@ -1230,15 +1232,16 @@ void plan_levels(als_solver* s) {
     const int dim = s->cfg.dimension;
     int lo[3] = {0, 0, 0};
     for (SolverLevel& L : s->levels) {
-        long long cells = 0, boxes = 0;
+        long long cells = 0, boxes = 0, tiles = 0;
         for (const SolverLevel& M : s->levels) {
             if (M.shape == L.shape) {
                 cells += region_cells(M.grid) * M.cfg.members;
-                boxes += face_boxes(M.grid, dim, s->cfg.precision) * M.cfg.members;
+                boxes += cover(M.grid, dim, als::kFacesKernel, s->cfg.precision) * M.cfg.members;
+                tiles += cover(M.grid, dim, 0, s->cfg.precision) * M.cfg.members;
             }
         }
         L.kernel = choose_kernel(dim, s->cfg.reconstruction, s->cfg.flux, L.shape, L.grid.n[0], cells,
-            boxes, s->cfg.precision);
+            boxes, tiles, s->cfg.precision);
         L.grid = make_grid(dim, L.grid.n, s->g, lo, L.grid.n, s->cfg.precision, L.kernel);
     }
     long long rows = 0, planes = 0;
@@ -1660,9 +1663,11 @@ int als_solver_advance(als_solver* s, long long steps) {
         const int cur0 = s->cur;
         ALS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
         int rc = ALS_OK;
+        s->capturing = true;
         for (int k = 0; k < per_graph && rc == ALS_OK; ++k) {
             rc = enqueue_step(s);
         }
+        s->capturing = false;
         cudaError_t err = cudaStreamEndCapture(s->stream, &g);
         s->cur = cur0;
         if (rc != ALS_OK) {

@@ -61,10 +61,15 @@ cudaError_t resident_blocks(int threads, size_t smem, int* blocks) {
 // (230 boxes of 296) 23 / 22; 24^3 29 / 33 (144 of 148); FP32 16 x 16 tiles 320^2 (400 of
 // 592) 27 / 30, 64 x 648 x 3 (492) 36 / 33.  Always chained: FP64 16 x 16 tiles (320^2 43 /
 // 41) and the FP32 1-D and 2-D faces, which are bound by latency, so that sharing an SM
-// costs them nothing (64^2: 18.2 / 17.5).
+// costs them nothing (64^2: 18.2 / 17.5).  These are replayed graphs; in steps launched one by
+// one (P.chained 2) the launch itself counts more, and all faces are chained (FP64, 4 steps:
+// 26 x 28 x 2 126 / 110 us, 61 x 339 106 / 93).
 template<void (*KERNEL)(StageParams)>
 cudaError_t launch_stage_blocks(int threads, size_t smem, const StageParams& P, int blocks_per_sm,
-    cudaStream_t stream, int quarters) {
+    cudaStream_t stream, int quarters, bool faces = false) {
+    if (faces && P.chained == 2) {
+        quarters = 0;
+    }
     // raising the dynamic shared-memory limit is idempotent and cheap; it is
     // done on every launch so that every device the process uses is covered
     cudaError_t err = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -117,11 +122,11 @@ cudaError_t launch_stage_one(const StageParams& P, int b, cudaStream_t s) {
     if constexpr (SHAPE == kFacesKernel) {
         typedef FaceLayout<R, DIM, RECON, FLUX> Lay;
         return launch_stage_blocks<faces_kernel<R, DIM, RECON, FLUX, KIND>>(Lay::THREADS, Lay::SMEM,
-            P, b, s, DIM == 3 ? 4 : (sizeof(R) == 4 ? 0 : 3));
+            P, b, s, DIM == 3 ? 4 : (sizeof(R) == 4 ? 0 : 3), true);
     } else if constexpr (SHAPE == kPlanesKernel) {
         typedef ZLayout<R, RECON, FLUX> Lay;
         return launch_stage_blocks<zmarch_kernel<R, RECON, FLUX, KIND>>(Lay::THREADS, Lay::SMEM, P,
-            b, s, 4);
+            b, s, 3);
     } else if constexpr (marches_rows(DIM, FLUX, SHAPE)) {
         typedef RowLayout<R, RECON, FLUX> Lay;
         // a block of the schedule stands for eight of these warps

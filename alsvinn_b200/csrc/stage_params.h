@@ -86,7 +86,7 @@ struct StageParams {
     int write_ghosts;        // 1: also write the boundary images of every updated cell
     double gamma;
     double c_fixed;          // dt/dx for stages when a level has no state
-    int chained;             // 1: a stage of the solver, launched while the one before it finishes
+    int chained;             // a stage of the solver, may be launched while the one before it ends: 1 in a graph, 2 by itself
     unsigned long long* counter; // persistent mode: [next item, blocks done], zero between launches; null: one item per block
 };
 

@@ -206,7 +206,7 @@ def test_uq_oracle_members_equal_single_runs_at_full_size(sample):
     assert y[0] == z["y"][sample]
 
 
-# above 100,000 cells in all, where shape 1 marches; ragged against the 16 x 15
+# above 400 tiles of 8 x 8 x 4 cells in all, where shape 1 marches; ragged against the 16 x 15
 # columns and the segments
 Z_CASES = [((41, 37, 34), "weno2", "hll3", "rungekutta3", "periodic", 2),
            ((33, 31, 100), "eno2", "hll", "rungekutta2", "neumann", 1),

@@ -33,8 +33,8 @@ CHOICES = [
     (3, (24, 24, 24), 1, "eno3", "hll3", "fp64", "faces"),           # 144
     (3, (28, 28, 28), 1, "eno3", "hll3", "fp64", "tiles"),
     (3, (28, 28, 28), 1, "weno2", "hll3", "fp32", "tiles"),
-    (3, (50, 50, 40), 1, "weno2", "hll3", "fp64", "tiles"),          # 100,000 cells
-    (3, (50, 50, 41), 1, "weno2", "hll3", "fp64", "columns"),
+    (3, (40, 40, 64), 1, "weno2", "hll3", "fp64", "tiles"),          # 400 tiles
+    (3, (40, 41, 56), 1, "weno2", "hll3", "fp64", "columns"),        # 420, fewer cells
     (3, (50, 50, 41), 1, "eno3", "hll3", "fp64", "tiles"),
     (1, (1024,), 1, "weno2", "hll", "fp64", "lines"),
     (1, (1024,), 4096, "weno2", "hll", "fp64", "lines"),             # several rounds
