@@ -401,7 +401,7 @@ namespace {
 // size: a cudaMalloc and cudaFree per accumulator cost more than adding a few hundred
 // states.  They are cudaMalloc's, so an accumulator's pointers (als_stats_moments) work with
 // peer access and cudaIpcGetMemHandle as any others; arrays whose pointers were handed out
-// are freed and not kept.  At most kKeptBytes per device, in arrays of up to kKeptArray;
+// are freed and not kept.  At most kKeptBytes per device, the latest, in arrays of up to kKeptArray;
 // als_scratch_trim and a failed allocation give them back.  A kept array is recognised by
 // its buffer id, which no other allocation ever has: one that a device reset took away is
 // forgotten.
@@ -431,9 +431,9 @@ unsigned long long buffer_id(const void* ptr) {
             CUDA_SUCCESS ? id : 0;
 }
 
-// Frees the current device's kept arrays down to `keep` bytes.
-void free_kept(int device, size_t keep) {
-    std::lock_guard<std::mutex> lock(g_kept_mutex);
+// Frees kept arrays of the current device, the longest kept first, down to
+// `keep` bytes; under g_kept_mutex.
+void free_kept_locked(int device, size_t keep) {
     size_t total = 0;
     for (const KeptArray& k : g_kept) {
         total += k.device == device ? k.bytes : 0;
@@ -449,6 +449,11 @@ void free_kept(int device, size_t keep) {
         total -= g_kept[i].bytes;
         g_kept.erase(g_kept.begin() + i);
     }
+}
+
+void free_kept(int device, size_t keep) {
+    std::lock_guard<std::mutex> lock(g_kept_mutex);
+    free_kept_locked(device, keep);
 }
 
 // `bytes` on the current device, kept or new.
@@ -482,14 +487,9 @@ void array_free(void* ptr, int device, size_t bytes, bool seen) {
     const unsigned long long id = seen || bytes > kKeptArray ? 0 : buffer_id(ptr);
     if (id) {
         std::lock_guard<std::mutex> lock(g_kept_mutex);
-        size_t total = bytes;
-        for (const KeptArray& k : g_kept) {
-            total += k.device == device ? k.bytes : 0;
-        }
-        if (total <= kKeptBytes) {
-            g_kept.push_back(KeptArray{device, ptr, bytes, id});
-            return;
-        }
+        free_kept_locked(device, kKeptBytes - bytes);
+        g_kept.push_back(KeptArray{device, ptr, bytes, id});
+        return;
     }
     cudaFree(ptr);
 }

@@ -63,6 +63,25 @@ def test_kept_arrays_start_from_zero_and_are_given_back():
     assert kept < after and after >= before
 
 
+def test_kept_arrays_are_the_latest_and_bounded():
+    """Sizes that never come back make room: after a dozen of them the arrays
+    of the last accumulator are kept (a new one of its size takes no memory), at
+    most 256 MiB in all."""
+    lib = als._lib.load()
+    torch.cuda.synchronize()
+    als._lib.check(lib.als_scratch_trim(0, 0))
+    start = torch.cuda.mem_get_info()[0]
+    for k in range(12):
+        als.MeanVariance(4000000 + 100000 * k).close()
+    full = torch.cuda.mem_get_info()[0]
+    assert start - full <= (256 + 16) << 20
+    mv = als.MeanVariance(4000000 + 100000 * 11)
+    assert torch.cuda.mem_get_info()[0] == full
+    mv.close()
+    als._lib.check(lib.als_scratch_trim(0, 0))
+    assert torch.cuda.mem_get_info()[0] >= start - (16 << 20)
+
+
 def test_seen_arrays_are_not_handed_to_the_next_accumulator():
     n = 1000003
     one = als.MeanVariance(n)
