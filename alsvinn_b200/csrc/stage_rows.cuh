@@ -16,7 +16,7 @@
 // So the reconstructed states and fluxes stay in registers, there is no
 // block barrier.  FP64 WENO2 + HLL3, per cell and stage: 670 to 701 FP64
 // instructions of 1,207 to 1,292 (the tiled kernel with plain divisions: 895 of
-// 2,650); FP64 pipe 55 to 58 % busy; FP32 642 to 750, 73 to 78 % of the issue
+// 2,650); FP64 pipe 55 to 58 % busy; FP32 620 to 710, 70 to 76 % of the issue
 // slots.  Ms per RK3 step: KH
 // 1024^2 FP64 0.279 (tiled) -> 0.235, 4096^2 4.66 (tiled, plain divisions) -> 2.83,
 // 512 x 256^2 FP32 members 4.35 -> 2.21.
